@@ -1008,27 +1008,40 @@ __device__ void hex_coefficients(const Box& bx, Exchange* h) {
     }
 }
 
+// Sum of a 64-bit integer over the warp, in every lane.
+__device__ __forceinline__ long long warp_sum(long long x) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+    return x;
+}
+
 // canon_force: forces from the list, stored; the closing half kick (not for
 // kPrime); the end-of-step sums in 32.32 fixed point, added per block, and in
 // the last block to finish the Nose-Hoover update or the exchange
 // coefficients.
+// The sums go through warp shuffles, one shared word per warp: shared memory
+// has no 64-bit add, so one atomicAdd per particle is a compare-and-swap loop
+// in which the whole block takes turns on one address (the exchange's pass
+// took 45 us that way at 2,462 atoms, 16.4 us so; Nose-Hoover's 18.5 us at
+// 15,600 atoms, 12.9 us so).
 template <bool SHIFTED_FORCE, int PASS>
 __global__ void __launch_bounds__(kForceThreads) canon_force_kernel(Arena a,
                                                                     const __grid_constant__ CUtensorMap map) {
     count_kernel(a);
+    constexpr int kWarps = kForceThreads / 32;
     __shared__ __align__(128) Stage st;
-    __shared__ unsigned long long s_sum[2][9];
+    __shared__ long long s_sum[kWarps][2][9];
     __shared__ int s_last;
     const uint32_t i = blockIdx.x * kForceThreads + threadIdx.x;
     const bool valid = i < a.nslots;
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     const Box& bx = a.boxes[0];
-    if (threadIdx.x < 18) s_sum[threadIdx.x / 9][threadIdx.x % 9] = 0ull;
     const PairSums s =
         block_pair_sums<SHIFTED_FORCE, false>(st, &map, a, bx, i, valid, a.cache[a.glob->phase]);
+    const float acc[3] = {s.ax, s.ay, s.az};
+    double v[3] = {0.0, 0.0, 0.0};
     if (valid) {
-        const float acc[3] = {s.ax, s.ay, s.az};
         a.acc[i] = make_float4(s.ax, s.ay, s.az, 0.0f);
-        double v[3];
 #pragma unroll
         for (int k = 0; k < 3; k++) {
             const size_t q = (size_t)k * a.seg + i;
@@ -1038,41 +1051,52 @@ __global__ void __launch_bounds__(kForceThreads) canon_force_kernel(Arena a,
                 a.v[q] = v[k];
             }
         }
-        const double es = (double)bx.energy_scale, ms = (double)bx.momentum_scale;
-        if (PASS == kPrime || PASS == kNoseHoover) {
-            const long long raw = fixed_raw_f64(0.5 * (v[0] * v[0] + v[1] * v[1] + v[2] * v[2]) * es);
-            if (raw) atomicAdd(&s_sum[0][0], (unsigned long long)raw);
-        }
-        if (PASS == kExchange) {
-            const int sl = hex_slab(bx, a.x[2 * (size_t)a.seg + i]);
-            if (sl < 2) {
-                unsigned long long* t = s_sum[sl];
-                atomicAdd(&t[0], 1ull << 32);
-                for (int k = 0; k < 3; k++) {
-                    atomicAdd(&t[1 + k], (unsigned long long)fixed_raw_f64(v[k] * ms));
-                    atomicAdd(&t[6 + k], (unsigned long long)fixed_raw_f64((double)acc[k] * ms));
-                }
-                atomicAdd(&t[4], (unsigned long long)fixed_raw_f64(
-                                     (v[0] * v[0] + v[1] * v[1] + v[2] * v[2]) * es));
-                atomicAdd(&t[5], (unsigned long long)fixed_raw_f64(
-                                     ((double)acc[0] * v[0] + (double)acc[1] * v[1] +
-                                      (double)acc[2] * v[2]) * es));
-            }
-        }
     }
     if (PASS == kKick) return;
+    const double es = (double)bx.energy_scale, ms = (double)bx.momentum_scale;
+    if (PASS == kExchange) {
+        const int sl = valid ? hex_slab(bx, a.x[2 * (size_t)a.seg + i]) : 2;
+#pragma unroll
+        for (int k = 0; k < 2; k++) {
+            const unsigned in = __ballot_sync(0xffffffffu, sl == k);
+            if (in == 0u) {
+                // most warps hold no particle of a slab
+                if (lane < 9u) s_sum[warp][k][lane] = 0ll;
+                continue;
+            }
+            long long raw[8];
+#pragma unroll
+            for (int c = 0; c < 3; c++) {
+                raw[c] = fixed_raw_f64(v[c] * ms);
+                raw[5 + c] = fixed_raw_f64((double)acc[c] * ms);
+            }
+            raw[3] = fixed_raw_f64((v[0] * v[0] + v[1] * v[1] + v[2] * v[2]) * es);
+            raw[4] = fixed_raw_f64(
+                ((double)acc[0] * v[0] + (double)acc[1] * v[1] + (double)acc[2] * v[2]) * es);
+            if (lane == 0) s_sum[warp][k][0] = (long long)__popc(in) << 32;
+#pragma unroll
+            for (int c = 0; c < 8; c++) {
+                const long long t = warp_sum(sl == k ? raw[c] : 0ll);
+                if (lane == 0) s_sum[warp][k][1 + c] = t;
+            }
+        }
+    } else {
+        const long long t =
+            warp_sum(valid ? fixed_raw_f64(0.5 * (v[0] * v[0] + v[1] * v[1] + v[2] * v[2]) * es) : 0ll);
+        if (lane == 0) s_sum[warp][0][0] = t;
+    }
+    __syncthreads();
+    if (threadIdx.x < (PASS == kExchange ? 18u : 1u)) {
+        const uint32_t sl = threadIdx.x / 9u, k = threadIdx.x % 9u;
+        long long t = 0;
+        for (int w = 0; w < kWarps; w++) t += s_sum[w][sl][k];
+        unsigned long long* to = PASS == kExchange ? &a.hex->sums[sl][k] : &a.nh->ke_raw;
+        if (t) atomicAdd(to, (unsigned long long)t);
+        __threadfence();
+    }
     __syncthreads();
     if (threadIdx.x == 0) {
-        uint32_t* done;
-        if (PASS == kExchange) {
-            for (int sl = 0; sl < 2; sl++)
-                for (int k = 0; k < 9; k++)
-                    if (s_sum[sl][k]) atomicAdd(&a.hex->sums[sl][k], s_sum[sl][k]);
-            done = &a.hex->blocks_done;
-        } else {
-            if (s_sum[0][0]) atomicAdd(&a.nh->ke_raw, s_sum[0][0]);
-            done = &a.nh->blocks_done;
-        }
+        uint32_t* done = PASS == kExchange ? &a.hex->blocks_done : &a.nh->blocks_done;
         __threadfence();
         s_last = atomicAdd(done, 1u) == gridDim.x - 1u;
     }
