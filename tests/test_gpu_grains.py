@@ -62,3 +62,12 @@ def test_loose_grains_with_crowded_contacts(gpu, O):
     radius = rng.uniform(0.0015, 0.0035, n)
     counts = run(gpu, O, pos, radius, box, 8)
     assert counts.max() > 8  # some grains have more contacts than the table holds
+
+
+@pytest.mark.parametrize("n", [1, 3, 10, 64, 65, 4097])
+def test_scan_runs_at_their_edges(gpu, O, n):
+    # 64^3 cells are 64 tiles of the prefix sum: fewer particles than tiles
+    # make its blocks take several tiles each, the last block a shorter run
+    rng = np.random.default_rng(n)
+    pos = rng.uniform(0.0, 1.0, (n, 3))
+    run(gpu, O, pos, rng.uniform(0.002, 0.007, n), 1.0, 4)
