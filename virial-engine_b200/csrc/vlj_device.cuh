@@ -32,13 +32,6 @@ __device__ __forceinline__ void count_kernel(const Arena& a) {
     if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&a.glob->kernels, 1ull);
 }
 
-// A step starts: the decision taken for it (if a step kernel took it) is
-// used up. Block 0 clears the flag before it counts itself finished, so the
-// last block's decision for the next step lands after the clear.
-__device__ __forceinline__ void consume_decision(const Arena& a) {
-    if (blockIdx.x == 0 && threadIdx.x == 0) a.glob->decided = 0u;
-}
-
 __device__ __forceinline__ bool rebuilding(const Arena& a, uint32_t b) {
     return a.ctrl[b].rebuild != 0u;
 }
@@ -151,14 +144,49 @@ __device__ __forceinline__ bool grid_pass(const Arena& a) {
 // With `set`, the decision (some box rebuilds) becomes the value of the graph
 // conditional `handle`.
 // A step kernel's last block takes the next step's decision itself
-// (`folded`) and leaves Global::decided set; the step that follows consumes
-// it (its step kernel clears the flag). A decide that finds such a decision
+// (`folded`: its own step is the one to finish) and leaves Global::decided
+// set until a step kernel that decides nothing clears it. A decide that finds such a decision
 // not yet consumed keeps it -- the displacements it came from were reset --
 // and only adds the boxes whose rebuild was forced since.
 __device__ __forceinline__ void decide_block(const Arena& a, cudaGraphConditionalHandle handle,
                                              bool set, bool folded = false) {
     __shared__ int s_any, s_keep;
     Global* g = a.glob;
+    if (folded && a.nboxes == 1u) {
+        // every other block has finished with these words: one thread reads
+        // them all at once and writes the outcome, a single round trip
+        if (threadIdx.x != 0) return;
+        Control& c = a.ctrl[0];
+        const Box& bx = a.boxes[0];
+        const uint32_t phase = g->phase, every = g->grid_every_step, built = c.built,
+                       forced = c.forced, rebuilds = c.rebuilds, moved = c.max_disp;
+        const unsigned long long step = g->step;
+        const bool rebuild = __uint_as_float(moved) > bx.half_skin2 || built == 0u || forced != 0u;
+        const bool grid = rebuild || every != 0u;
+        const uint32_t n = grid ? bx.n : 0u;
+        g->phase = phase ^ 1u;
+        g->step = step + 1ull;
+        g->decided = 1u;
+        g->work_front = 0u;
+        g->work_back = 0u;
+        g->next_build = 0u;
+        c.max_disp = 0u;
+        c.forced = 0u;
+        c.rebuild = rebuild ? 1u : 0u;
+        c.reorder = rebuild && rebuilds % bx.reorder_every == 0u ? 1u : 0u;
+        if (rebuild) {
+            c.rebuilds = rebuilds + 1u;
+            c.built = 1u;
+        }
+        a.rb_box[0] = 0u;
+        a.rb_first[0] = 0u;
+        a.rb_first[grid ? 1 : 0] = n;
+        g->rb_boxes = grid ? 1u : 0u;
+        g->rb_slots = n;
+        g->any = rebuild ? 1u : 0u;
+        if (set) cudaGraphSetConditional(handle, rebuild ? 1u : 0u);
+        return;
+    }
     if (threadIdx.x == 0) {
         s_any = 0;
         s_keep = !folded && g->decided != 0u;
@@ -166,7 +194,7 @@ __device__ __forceinline__ void decide_block(const Arena& a, cudaGraphConditiona
         g->work_front = 0u;
         g->work_back = 0u;
         g->next_build = 0u;
-        if (g->pending) {
+        if (folded || g->pending) {
             g->phase ^= 1u;
             g->step += 1ull;
             g->pending = 0u;
@@ -313,27 +341,22 @@ __device__ __forceinline__ bool block_in_one_box(const Arena& a, bool valid, uin
     return s_mixed == 0;
 }
 
-// Largest value over the block into each box's max_disp: one atomicMax when
-// the block lies in one box (the usual case), one per thread otherwise.
-__device__ __forceinline__ void block_max_per_box(const Arena& a, bool valid, uint32_t b,
-                                                  uint32_t first_slot, float value) {
-    __shared__ uint32_t s_val[kBlock / 32];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    uint32_t bits = valid ? __float_as_uint(value) : 0u;
-    uint32_t ref;
-    if (!block_in_one_box(a, valid, b, first_slot, &ref)) {
-        if (valid) atomicMax(&a.ctrl[b].max_disp, bits);
-        return;
+// A particle's squared displacement since the last list build: into its box's
+// max_disp where it is past the rebuild trigger (the decision asks no more of
+// it, and on most steps nothing is), one atomic a warp when the warp lies in
+// one box. Returns whether this thread's was past it. Every lane must call.
+__device__ __forceinline__ bool note_displacement(const Arena& a, bool valid, uint32_t b, float value) {
+    const bool over = valid && value > a.boxes[b].half_skin2;
+    if (!__any_sync(0xffffffffu, over)) return false;
+    const uint32_t bits = over ? __float_as_uint(value) : 0u;
+    const uint32_t first = __shfl_sync(0xffffffffu, b, __ffs(__ballot_sync(0xffffffffu, over)) - 1);
+    if (__all_sync(0xffffffffu, !over || b == first)) {
+        const uint32_t m = __reduce_max_sync(0xffffffffu, bits);
+        if ((threadIdx.x & 31u) == 0u) atomicMax(&a.ctrl[first].max_disp, m);
+    } else if (over) {
+        atomicMax(&a.ctrl[b].max_disp, bits);
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) bits = max(bits, __shfl_xor_sync(0xffffffffu, bits, o));
-    if (lane == 0) s_val[warp] = bits;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        uint32_t m = 0;
-        for (int w = 0; w < (int)(blockDim.x >> 5); w++) m = max(m, s_val[w]);
-        atomicMax(&a.ctrl[ref].max_disp, m);
-    }
+    return true;
 }
 
 // Sum of kSlots 64-bit integers over the block into each box's accumulators,

@@ -26,12 +26,11 @@ constexpr uint32_t kTileBytes = kTileRows * kForceThreads * 16u;
 #define VLJ_STEP_MIN_BLOCKS 1
 #endif
 constexpr int kStepMinBlocks = VLJ_STEP_MIN_BLOCKS;
-// Grids of at most this many blocks (of one particle a thread) per SM step
-// with two lanes per particle (step_kernel_split).
-#ifndef VLJ_SPLIT_BLOCKS_PER_SM
-#define VLJ_SPLIT_BLOCKS_PER_SM 4
+// Lanes per particle of the force kernels, by grid size (lanes_for): at most
+// this many threads per SM after the split.
+#ifndef VLJ_LANE_THREADS_PER_SM
+#define VLJ_LANE_THREADS_PER_SM 512
 #endif
-constexpr int kSplitBlocksPerSM = VLJ_SPLIT_BLOCKS_PER_SM;
 constexpr unsigned long long kWaitLimitNs = 500000000ull;  // 0.5 s per TMA tile
 
 struct PairSums {
@@ -42,32 +41,24 @@ struct PairSums {
     // heat current: half of the pair energies, and T = sum_j d d^T |F| / r
     // (xx yy zz xy xz yz)
     float e_half, t[6];
-    // The force is summed in two parts, the entries of the list's even rows
-    // (ax, ay, az) and of its odd rows (these), added once at the end
-    // (combine_parts): one thread walking all rows and two lanes walking
-    // half of them each then give the same bits.
-    float ax1, ay1, az1;
+    // The force is summed in parts of two list rows (eight entries): each
+    // part's sum starts from zero (px, py, pz) and joins the total (ax, ay,
+    // az) in list order (end_part). One thread walking all rows and several
+    // lanes taking a part each then give the same bits.
+    float px, py, pz;
 };
 
-__device__ __forceinline__ void combine_parts(PairSums& s) {
-    s.ax = __fadd_rn(s.ax, s.ax1);
-    s.ay = __fadd_rn(s.ay, s.ay1);
-    s.az = __fadd_rn(s.az, s.az1);
-    s.ax1 = s.ay1 = s.az1 = 0.0f;
+__device__ __forceinline__ void end_part(PairSums& s) {
+    s.ax = __fadd_rn(s.ax, s.px);
+    s.ay = __fadd_rn(s.ay, s.py);
+    s.az = __fadd_rn(s.az, s.pz);
+    s.px = s.py = s.pz = 0.0f;
 }
 
-// the force part of the list's row parity PART
-template <int PART>
 __device__ __forceinline__ void add_force(PairSums& s, float dx, float dy, float dz, float f) {
-    if (PART == 0) {
-        s.ax = __fmaf_rn(-dx, f, s.ax);
-        s.ay = __fmaf_rn(-dy, f, s.ay);
-        s.az = __fmaf_rn(-dz, f, s.az);
-    } else {
-        s.ax1 = __fmaf_rn(-dx, f, s.ax1);
-        s.ay1 = __fmaf_rn(-dy, f, s.ay1);
-        s.az1 = __fmaf_rn(-dz, f, s.az1);
-    }
+    s.px = __fmaf_rn(-dx, f, s.px);
+    s.py = __fmaf_rn(-dy, f, s.py);
+    s.pz = __fmaf_rn(-dz, f, s.pz);
 }
 
 // Shared memory of a force-kernel block: the tile ring and its barriers
@@ -152,7 +143,7 @@ __device__ __forceinline__ bool bar_wait(unsigned long long* bar, uint32_t parit
 // the halves of the pair energy and virial as unevaluated f32 pairs (as the
 // reference sums them in double-float, lennard_jones.wgsl:518-519). A zero
 // separation (the padding of a list's last row) adds nothing.
-template <bool SHIFTED_FORCE, bool ENERGIES, bool HEAT, int PART = 0>
+template <bool SHIFTED_FORCE, bool ENERGIES, bool HEAT>
 __device__ __forceinline__ void pair_terms(PairSums& s, const uint4 own, const uint4 pj,
                                            const Box& bx, float dec0, float dec1, float dec2,
                                            uint32_t rc2_bits_m1, float fshift) {
@@ -164,7 +155,7 @@ __device__ __forceinline__ void pair_terms(PairSums& s, const uint4 own, const u
     // branch-free: most list entries are inside the cutoff; the select
     // drops whatever the pair math gives for entries that are not
     const float f = in ? lj_force_over_r2<SHIFTED_FORCE>(r2, fshift) : 0.0f;
-    add_force<PART>(s, dx, dy, dz, f);
+    add_force(s, dx, dy, dz, f);
     if (HEAT) {
         s.e_half += in ? 0.5f * lj_energy_fast<SHIFTED_FORCE>(r2, bx) : 0.0f;
         const float fx = dx * f, fy = dy * f, fz = dz * f;
@@ -197,7 +188,7 @@ __device__ __forceinline__ void pair_terms(PairSums& s, const uint4 own, const u
 
 // pair_terms on positions given as f32 offsets from a common origin near
 // both (the cell tiles' f32 form): the separation is their plain difference.
-template <bool SHIFTED_FORCE, bool HEAT, int PART = 0>
+template <bool SHIFTED_FORCE, bool HEAT>
 __device__ __forceinline__ void pair_terms_rel(PairSums& s, const float4 own, const float4 pj,
                                                const Box& bx, uint32_t rc2_bits_m1, float fshift) {
     const float dx = __fsub_rn(pj.x, own.x);
@@ -206,7 +197,7 @@ __device__ __forceinline__ void pair_terms_rel(PairSums& s, const float4 own, co
     const float r2 = sep_r2(dx, dy, dz);
     const bool in = __float_as_uint(r2) - 1u < rc2_bits_m1;
     const float f = in ? lj_force_over_r2<SHIFTED_FORCE>(r2, fshift) : 0.0f;
-    add_force<PART>(s, dx, dy, dz, f);
+    add_force(s, dx, dy, dz, f);
     if (HEAT) {
         s.e_half += in ? 0.5f * lj_energy_fast<SHIFTED_FORCE>(r2, bx) : 0.0f;
         const float fx = dx * f, fy = dy * f, fz = dz * f;
@@ -257,28 +248,18 @@ __device__ __forceinline__ PairSums block_pair_sums(Stage& st, const CUtensorMap
     const uint32_t rc2_bits_m1 = __float_as_uint(rc2) - 1u;
     // The list's last row is padded with the particle itself, whose zero
     // separation drops out with the entries beyond the cutoff.
-    auto acc0 = [&](const uint4 pj) {
-        pair_terms<SHIFTED_FORCE, ENERGIES, HEAT, 0>(s, own, pj, bx, dec0, dec1, dec2,
-                                                     rc2_bits_m1, fshift);
+    auto add = [&](const uint4 pj) {
+        pair_terms<SHIFTED_FORCE, ENERGIES, HEAT>(s, own, pj, bx, dec0, dec1, dec2,
+                                                  rc2_bits_m1, fshift);
     };
-    auto acc1 = [&](const uint4 pj) {
-        pair_terms<SHIFTED_FORCE, ENERGIES, HEAT, 1>(s, own, pj, bx, dec0, dec1, dec2,
-                                                     rc2_bits_m1, fshift);
-    };
-    // the four entries of list row `row`, into the force part of its parity
+    // the four entries of list row `row`; a part ends with its odd row
     auto row_terms = [&](uint32_t row, const uint4 p0, const uint4 p1, const uint4 p2,
                          const uint4 p3) {
-        if (row & 1u) {
-            acc1(p0);
-            acc1(p1);
-            acc1(p2);
-            acc1(p3);
-        } else {
-            acc0(p0);
-            acc0(p1);
-            acc0(p2);
-            acc0(p3);
-        }
+        add(p0);
+        add(p1);
+        add(p2);
+        add(p3);
+        if (row & 1u) end_part(s);
     };
 
 #if VLJ_LIST_STREAM
@@ -310,7 +291,7 @@ __device__ __forceinline__ PairSums block_pair_sums(Stage& st, const CUtensorMap
     }
 #else
     // each thread its own rows, the next one in flight while it works on
-    // this; two rows an iteration, the even one's force part then the odd's
+    // this; two rows an iteration: a part of the force sum
     uint4 next = my_rows ? load_row_streaming(rowp) : make_uint4(0u, 0u, 0u, 0u);
     for (uint32_t row = 0; row < my_rows; row += 2u) {
         {
@@ -320,10 +301,10 @@ __device__ __forceinline__ PairSums block_pair_sums(Stage& st, const CUtensorMap
             const uint4 p1 = __ldg(cur + e.y);
             const uint4 p2 = __ldg(cur + e.z);
             const uint4 p3 = __ldg(cur + e.w);
-            acc0(p0);
-            acc0(p1);
-            acc0(p2);
-            acc0(p3);
+            add(p0);
+            add(p1);
+            add(p2);
+            add(p3);
         }
         if (row + 1u < my_rows) {
             const uint4 e = next;
@@ -332,14 +313,15 @@ __device__ __forceinline__ PairSums block_pair_sums(Stage& st, const CUtensorMap
             const uint4 p1 = __ldg(cur + e.y);
             const uint4 p2 = __ldg(cur + e.z);
             const uint4 p3 = __ldg(cur + e.w);
-            acc1(p0);
-            acc1(p1);
-            acc1(p2);
-            acc1(p3);
+            add(p0);
+            add(p1);
+            add(p2);
+            add(p3);
+            end_part(s);
         }
     }
 #endif
-    combine_parts(s);
+    end_part(s);
     return s;
 #else
     bool lost = false;
@@ -380,9 +362,55 @@ __device__ __forceinline__ PairSums block_pair_sums(Stage& st, const CUtensorMap
         }
         __syncthreads();
     }
-    combine_parts(s);
+    end_part(s);
     return s;
 #endif
+}
+
+// The force on particle i (all components in every lane) with LANES
+// consecutive threads sharing its list: in each round lane `sub` sums part
+// round * LANES + sub (two rows, eight gathers in flight), and the round's
+// parts join the total in list order, so the bits are block_pair_sums's. The
+// next round's rows load behind this one's pairs. A row past the list's end
+// reads as the particle itself, whose zero separation adds nothing. Every
+// lane of the warp must call this.
+template <bool SHIFTED_FORCE, int LANES>
+__device__ __forceinline__ void lane_forces(const Arena& a, const Box& bx, uint32_t i, bool valid,
+                                            uint32_t sub, const uint4* __restrict__ cur,
+                                            float (&f)[3]) {
+    const uint32_t at = valid ? i : 0u;
+    const uint4 own = __ldg(cur + at);
+    const uint32_t rows = valid ? (__ldg(a.list_count + at) + 3u) / 4u : 0u;
+    const uint32_t rounds =
+        __reduce_max_sync(0xffffffffu, (rows + 2u * LANES - 1u) / (2u * LANES));
+    const float dec0 = bx.dec[0], dec1 = bx.dec[1], dec2 = bx.dec[2];
+    const float fshift = bx.force_shift;
+    const uint32_t rc2_bits_m1 = __float_as_uint(bx.rc2) - 1u;
+    const uint4* rowp = reinterpret_cast<const uint4*>(a.list) + at;
+    const uint4 self = make_uint4(at, at, at, at);
+    uint32_t row = 2u * sub;
+    uint4 e0 = row < rows ? load_row_streaming(rowp + (size_t)row * a.seg) : self;
+    uint4 e1 = row + 1u < rows ? load_row_streaming(rowp + (size_t)(row + 1u) * a.seg) : self;
+    f[0] = f[1] = f[2] = 0.0f;
+    for (uint32_t r = 0; r < rounds; r++) {
+        const uint4 p[8] = {__ldg(cur + e0.x), __ldg(cur + e0.y), __ldg(cur + e0.z), __ldg(cur + e0.w),
+                            __ldg(cur + e1.x), __ldg(cur + e1.y), __ldg(cur + e1.z), __ldg(cur + e1.w)};
+        row += 2u * LANES;
+        e0 = row < rows ? load_row_streaming(rowp + (size_t)row * a.seg) : self;
+        e1 = row + 1u < rows ? load_row_streaming(rowp + (size_t)(row + 1u) * a.seg) : self;
+        PairSums s = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0u,
+                      0.0f, {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f}};
+#pragma unroll
+        for (int k = 0; k < 8; k++)
+            pair_terms<SHIFTED_FORCE, false, false>(s, own, p[k], bx, dec0, dec1, dec2, rc2_bits_m1,
+                                                    fshift);
+#pragma unroll
+        for (int k = 0; k < LANES; k++) {
+            f[0] = __fadd_rn(f[0], __shfl_sync(0xffffffffu, s.px, k, LANES));
+            f[1] = __fadd_rn(f[1], __shfl_sync(0xffffffffu, s.py, k, LANES));
+            f[2] = __fadd_rn(f[2], __shfl_sync(0xffffffffu, s.pz, k, LANES));
+        }
+    }
 }
 
 // Sum of one heat-current sample's three components over the block into
@@ -448,6 +476,33 @@ __device__ __forceinline__ void heat_terms(const Arena& a, const Box& bx, uint32
     for (int c = 0; c < 3; c++) raw[c] += fixed_raw_f64(e * v[c] + 0.5 * tv[c]);
 }
 
+// Component c of langevin_noise alone.
+__device__ __forceinline__ float langevin_noise_of(uint32_t c, uint32_t id, unsigned long long step,
+                                                   uint32_t seed) {
+    const uint4 r = philox(id, step, seed);
+    const float scale = 5.9604644775390625e-08f;  // 2^-24
+    const float u = ((float)((c < 2u ? r.x : r.z) >> 8) + 1.0f) * scale;
+    const float t = ((float)((c < 2u ? r.y : r.w) >> 8) + 1.0f) * scale;
+    const float radius = sqrtf(-2.0f * logf(u));
+    const float angle = 6.283185307179586f * t;
+    return radius * (c == 1u ? sinf(angle) : cosf(angle));
+}
+
+// One component's step: both half kicks, then the drift. Every operation
+// spelled out, so each kernel gets the same bits.
+__device__ __forceinline__ void advance_component(const Box& bx, double side, float acc, float xi,
+                                                  double& x, double& v) {
+    v = __fma_rn((double)acc, bx.dt, v);
+    if (bx.thermostat == 1) {
+        x = __fma_rn(v, bx.half_dt, x);
+        v = __fma_rn(bx.c1, v, __dmul_rn(bx.c2, (double)xi));
+        x = __fma_rn(v, bx.half_dt, x);
+    } else {
+        x = __fma_rn(v, bx.dt, x);
+    }
+    x = wrap(x, side);
+}
+
 // begin + force_kick of the reference for slot i (lennard_jones.wgsl:204-276,
 // 556-574), with its forces in s: the stored velocity is half a kick behind,
 // so the two half kicks go on together, then the drift: x += v dt (constant
@@ -468,24 +523,48 @@ __device__ __forceinline__ float advance_slot(const Arena& a, const Box& bx, uin
 #pragma unroll
     for (int k = 0; k < 3; k++) {
         const size_t q = (size_t)k * a.seg + i;
-        double x = a.x[q];
-        double v = a.v[q] + (double)acc[k] * bx.dt;
-        if (langevin) {
-            x += v * bx.half_dt;
-            v = bx.c1 * v + bx.c2 * (double)xi[k];
-            x += v * bx.half_dt;
-        } else {
-            x += v * bx.dt;
-        }
-        x = wrap(x, bx.box[k]);
+        double x = a.x[q], v = a.v[q];
+        advance_component(bx, bx.box[k], acc[k], xi[k], x, v);
         a.x[q] = x;
         a.v[q] = v;
         enc[k] = encode(x, bx.enc[k]);
         const float d = decode_diff(enc[k], sw[k], bx.dec[k]);
-        disp2 += d * d;
+        disp2 = __fmaf_rn(d, d, disp2);
     }
     a.cache[phase ^ 1u][i] = make_uint4(enc[0], enc[1], enc[2], 0u);
     return disp2;
+}
+
+// The end of a step kernel: the displacement trigger, then, with `next` (or
+// a heat-current sample taken), the last block to finish takes the next
+// step's rebuild decision and moves the heat-current series on. Called by
+// every thread of the block. Only a displacement past the trigger is written
+// (the decision asks for no more), so on most steps the block's count is the
+// one global round trip, with no fence to wait for.
+template <bool HEAT>
+__device__ __forceinline__ void finish_step(const Arena& a, bool valid, uint32_t b, float disp2,
+                                            cudaGraphConditionalHandle next) {
+    const bool over = note_displacement(a, valid, b, disp2);
+    if (!next && blockIdx.x == 0 && threadIdx.x == 0) {
+        // the next decide finishes this step, and decides anew
+        a.glob->pending = 1u;
+        a.glob->decided = 0u;
+    }
+    if (!next && !HEAT) return;
+    __shared__ int s_last;
+    const int any_over = __syncthreads_or(over);
+    if (threadIdx.x == 0) {
+        if (any_over) __threadfence();
+        s_last = atomicAdd(&a.glob->blocks_done, 1u) == gridDim.x - 1u;
+    }
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    if (threadIdx.x == 0) {
+        a.glob->blocks_done = 0u;
+        if (HEAT) a.glob->heat_next += 1u;
+    }
+    if (next) decide_block(a, next, true, true);
 }
 
 // ---- prime (lennard_jones.wgsl:547-553): first forces; the stored velocity
@@ -536,7 +615,6 @@ __global__ void __launch_bounds__(THREADS, kStepMinBlocks) step_kernel(Arena a,
                                                              cudaGraphConditionalHandle next) {
     static_assert(VLJ_LIST_STREAM || THREADS == kForceThreads, "TMA tiles need kForceThreads");
     count_kernel(a);
-    consume_decision(a);
     __shared__ __align__(128) Stage st;
 #if VLJ_STEP_REMAP
     const uint32_t vb = resident_neighbours(blockIdx.x, gridDim.x, a.remap_sms, a.remap_per_sm);
@@ -558,93 +636,61 @@ __global__ void __launch_bounds__(THREADS, kStepMinBlocks) step_kernel(Arena a,
     }
     float disp2 = 0.0f;
     if (valid) disp2 = advance_slot(a, bx, i, phase, s);
-    block_max_per_box(a, valid, b, vb * THREADS, disp2);
-    if (i == 0) a.glob->pending = 1u;
-    if (!next && !HEAT) return;
-    // the last block to finish takes the next step's rebuild decision and
-    // moves the heat-current series on
-    __shared__ int s_last;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        __threadfence();
-        s_last = atomicAdd(&a.glob->blocks_done, 1u) == gridDim.x - 1u;
-    }
-    __syncthreads();
-    if (!s_last) return;
-    __threadfence();
-    if (threadIdx.x == 0) {
-        a.glob->blocks_done = 0u;
-        if (HEAT) a.glob->heat_next += 1u;
-    }
-    if (next) decide_block(a, next, true, true);
+    finish_step<HEAT>(a, valid, b, disp2, next);
 }
 
-// ---- one step with two lanes per particle, for grids of a few blocks per
-// SM (small boxes), whose lone warps cannot hide their latency behind each
-// other's: lane h of a pair walks the particle's list rows h, h + 2, ...
-// into one force part, the pair adds the two parts as combine_parts does
-// (even rows' first), and lane 0 integrates. The same step as step_kernel
-// to the bit (no heat-current sample). ----
-template <bool SHIFTED_FORCE, int THREADS>
-__global__ void __launch_bounds__(THREADS) step_kernel_split(Arena a, cudaGraphConditionalHandle next) {
+// ---- one step with LANES lanes per particle, for grids that leave the chip
+// idle at one (lanes_for): a lone warp cannot hide its latency behind others,
+// so its chain of rows and gathers is what the step takes. The list's parts
+// go to the lanes (lane_forces); with four lanes or more, lane c < 3 then
+// steps component c, its state loaded before the forces. The same step as
+// step_kernel to the bit (no heat-current sample). ----
+template <bool SHIFTED_FORCE, int LANES, int THREADS>
+__global__ void __launch_bounds__(THREADS) step_kernel_lanes(Arena a, cudaGraphConditionalHandle next) {
     count_kernel(a);
-    consume_decision(a);
-    constexpr uint32_t kPer = THREADS / 2;  // particles per block
-    const uint32_t h = threadIdx.x & 1u;
-    const uint32_t i = blockIdx.x * kPer + (threadIdx.x >> 1);
+    constexpr uint32_t kPer = THREADS / LANES;  // particles per block
+    const uint32_t sub = threadIdx.x % LANES;
+    const uint32_t i = blockIdx.x * kPer + threadIdx.x / LANES;
     const bool valid = i < a.nslots;
     const uint32_t phase = a.glob->phase;
     const uint32_t b = valid ? box_of_slot(a, i) : 0u;
     const Box& bx = a.boxes[b];
-    const uint4* __restrict__ cur = a.cache[phase];
-    PairSums s = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0u,
-                  0.0f, {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f}};
-    if (valid) {
-        const uint4 own = __ldg(cur + i);
-        const uint32_t rows = (__ldg(a.list_count + i) + 3u) / 4u;
-        const float dec0 = bx.dec[0], dec1 = bx.dec[1], dec2 = bx.dec[2];
-        const float fshift = bx.force_shift;
-        const uint32_t rc2_bits_m1 = __float_as_uint(bx.rc2) - 1u;
-        const uint4* rowp = reinterpret_cast<const uint4*>(a.list) + i;
-        uint4 nxt = h < rows ? load_row_streaming(rowp + (size_t)h * a.seg) : make_uint4(0u, 0u, 0u, 0u);
-        for (uint32_t row = h; row < rows; row += 2u) {
-            const uint4 e = nxt;
-            if (row + 2u < rows) nxt = load_row_streaming(rowp + (size_t)(row + 2u) * a.seg);
-            const uint4 p0 = __ldg(cur + e.x);
-            const uint4 p1 = __ldg(cur + e.y);
-            const uint4 p2 = __ldg(cur + e.z);
-            const uint4 p3 = __ldg(cur + e.w);
-            pair_terms<SHIFTED_FORCE, false, false, 0>(s, own, p0, bx, dec0, dec1, dec2, rc2_bits_m1, fshift);
-            pair_terms<SHIFTED_FORCE, false, false, 0>(s, own, p1, bx, dec0, dec1, dec2, rc2_bits_m1, fshift);
-            pair_terms<SHIFTED_FORCE, false, false, 0>(s, own, p2, bx, dec0, dec1, dec2, rc2_bits_m1, fshift);
-            pair_terms<SHIFTED_FORCE, false, false, 0>(s, own, p3, bx, dec0, dec1, dec2, rc2_bits_m1, fshift);
+    float f[3];
+    if constexpr (LANES >= 4) {
+        const bool mine = valid && sub < 3u;
+        const size_t q = (size_t)sub * a.seg + i;
+        double x = 0.0, v = 0.0;
+        uint32_t sw = 0, id = 0;
+        if (mine) {
+            x = a.x[q];
+            v = a.v[q];
+            sw = reinterpret_cast<const uint32_t*>(a.snap + i)[sub];
+            if (bx.thermostat == 1) id = a.id[i];
         }
+        lane_forces<SHIFTED_FORCE, LANES>(a, bx, i, valid, sub, a.cache[phase], f);
+        float d = 0.0f;
+        if (mine) {
+            const float xi = bx.thermostat == 1 ? langevin_noise_of(sub, id, a.glob->step, bx.seed) : 0.0f;
+            advance_component(bx, bx.box[sub], sub == 0u ? f[0] : (sub == 1u ? f[1] : f[2]), xi, x, v);
+            a.x[q] = x;
+            a.v[q] = v;
+            const uint32_t enc = encode(x, bx.enc[sub]);
+            d = decode_diff(enc, sw, bx.dec[sub]);
+            reinterpret_cast<uint32_t*>(a.cache[phase ^ 1u] + i)[sub] = enc;
+        }
+        float disp2 = 0.0f;
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            const float dk = __shfl_sync(0xffffffffu, d, k, LANES);
+            disp2 = __fmaf_rn(dk, dk, disp2);
+        }
+        finish_step<false>(a, valid, b, disp2, next);
+    } else {
+        lane_forces<SHIFTED_FORCE, LANES>(a, bx, i, valid, sub, a.cache[phase], f);
+        const PairSums s = {f[0], f[1], f[2]};
+        const bool mine = valid && sub == 0u;
+        finish_step<false>(a, mine, b, mine ? advance_slot(a, bx, i, phase, s) : 0.0f, next);
     }
-    // lane 0 holds the even rows' part, lane 1 the odd rows'
-    const float ox = __shfl_xor_sync(0xffffffffu, s.ax, 1);
-    const float oy = __shfl_xor_sync(0xffffffffu, s.ay, 1);
-    const float oz = __shfl_xor_sync(0xffffffffu, s.az, 1);
-    s.ax = __fadd_rn(s.ax, ox);
-    s.ay = __fadd_rn(s.ay, oy);
-    s.az = __fadd_rn(s.az, oz);
-    const bool mine = valid && h == 0u;
-    float disp2 = 0.0f;
-    if (mine) disp2 = advance_slot(a, bx, i, phase, s);
-    block_max_per_box(a, mine, b, blockIdx.x * kPer, disp2);
-    if (i == 0 && h == 0u) a.glob->pending = 1u;
-    if (!next) return;
-    // the last block to finish takes the next step's rebuild decision
-    __shared__ int s_last;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        __threadfence();
-        s_last = atomicAdd(&a.glob->blocks_done, 1u) == gridDim.x - 1u;
-    }
-    __syncthreads();
-    if (!s_last) return;
-    __threadfence();
-    if (threadIdx.x == 0) a.glob->blocks_done = 0u;
-    decide_block(a, next, true, true);
 }
 
 // ---- one step over cell tiles: the same step as step_kernel, with the
@@ -662,7 +708,6 @@ __global__ void __launch_bounds__(THREADS) step_kernel_split(Arena a, cudaGraphC
 template <bool SHIFTED_FORCE, bool HEAT>
 __global__ void __launch_bounds__(kBlock) tile_step_kernel(Arena a, cudaGraphConditionalHandle next) {
     count_kernel(a);
-    consume_decision(a);
     extern __shared__ __align__(16) uint4 s_tile[];
     __shared__ uint32_t s_run[9][3];  // per tile row: first run's sorted start, its length, second run's start
     __shared__ uint32_t s_base[10];   // tile index of each row's first particle; [9]: the tile's size
@@ -738,25 +783,17 @@ __global__ void __launch_bounds__(kBlock) tile_step_kernel(Arena a, cudaGraphCon
         if (staged) {
 #if VLJ_TILE_F32
             const float4 own = s_tilef[own0 + p];
-            // a 16-bit row's first four entries are a slot-list row of even
-            // index (add0), its last four one of odd index (add1)
-            auto add0 = [&](const float4 pj) {
-                pair_terms_rel<SHIFTED_FORCE, HEAT, 0>(s, own, pj, bx, rc2_bits_m1, fshift);
-            };
-            auto add1 = [&](const float4 pj) {
-                pair_terms_rel<SHIFTED_FORCE, HEAT, 1>(s, own, pj, bx, rc2_bits_m1, fshift);
+            // a 16-bit row is two rows of the slot list: a part of the force sum
+            auto add = [&](const float4 pj) {
+                pair_terms_rel<SHIFTED_FORCE, HEAT>(s, own, pj, bx, rc2_bits_m1, fshift);
             };
             auto fetch = [&](uint32_t t) { return s_tilef[t]; };
             using Pos = float4;
 #else
             const uint4 own = s_tile[own0 + p];
-            auto add0 = [&](const uint4 pj) {
-                pair_terms<SHIFTED_FORCE, false, HEAT, 0>(s, own, pj, bx, dec0, dec1, dec2,
-                                                          rc2_bits_m1, fshift);
-            };
-            auto add1 = [&](const uint4 pj) {
-                pair_terms<SHIFTED_FORCE, false, HEAT, 1>(s, own, pj, bx, dec0, dec1, dec2,
-                                                          rc2_bits_m1, fshift);
+            auto add = [&](const uint4 pj) {
+                pair_terms<SHIFTED_FORCE, false, HEAT>(s, own, pj, bx, dec0, dec1, dec2,
+                                                       rc2_bits_m1, fshift);
             };
             auto fetch = [&](uint32_t t) { return s_tile[t]; };
             using Pos = uint4;
@@ -789,22 +826,22 @@ __global__ void __launch_bounds__(kBlock) tile_step_kernel(Arena a, cudaGraphCon
                     q[6] = fetch(e.w & 0xffffu); q[7] = fetch(e.w >> 16);
                 }
 #pragma unroll
-                for (int m = 0; m < 4; m++) add0(c[m]);
-#pragma unroll
-                for (int m = 4; m < 8; m++) add1(c[m]);
+                for (int m = 0; m < 8; m++) add(c[m]);
+                end_part(s);
             }
 #else
             for (uint32_t row = 0; row < rows; row++) {
                 const uint4 e = nxt;
                 if (row + 1u < rows) nxt = load_row_streaming(rowp + (size_t)(row + 1u) * a.seg);
-                add0(fetch(e.x & 0xffffu));
-                add0(fetch(e.x >> 16));
-                add0(fetch(e.y & 0xffffu));
-                add0(fetch(e.y >> 16));
-                add1(fetch(e.z & 0xffffu));
-                add1(fetch(e.z >> 16));
-                add1(fetch(e.w & 0xffffu));
-                add1(fetch(e.w >> 16));
+                add(fetch(e.x & 0xffffu));
+                add(fetch(e.x >> 16));
+                add(fetch(e.y & 0xffffu));
+                add(fetch(e.y >> 16));
+                add(fetch(e.z & 0xffffu));
+                add(fetch(e.z >> 16));
+                add(fetch(e.w & 0xffffu));
+                add(fetch(e.w >> 16));
+                end_part(s);
             }
 #endif
         } else {
@@ -815,43 +852,17 @@ __global__ void __launch_bounds__(kBlock) tile_step_kernel(Arena a, cudaGraphCon
                 const uint4 e = load_row_streaming(rowp + (size_t)row * a.seg);
                 const uint4 p0 = __ldg(cur + e.x), p1 = __ldg(cur + e.y);
                 const uint4 p2 = __ldg(cur + e.z), p3 = __ldg(cur + e.w);
-                if (row & 1u) {
-                    pair_terms<SHIFTED_FORCE, false, HEAT, 1>(s, own, p0, bx, dec0, dec1, dec2, rc2_bits_m1, fshift);
-                    pair_terms<SHIFTED_FORCE, false, HEAT, 1>(s, own, p1, bx, dec0, dec1, dec2, rc2_bits_m1, fshift);
-                    pair_terms<SHIFTED_FORCE, false, HEAT, 1>(s, own, p2, bx, dec0, dec1, dec2, rc2_bits_m1, fshift);
-                    pair_terms<SHIFTED_FORCE, false, HEAT, 1>(s, own, p3, bx, dec0, dec1, dec2, rc2_bits_m1, fshift);
-                } else {
-                    pair_terms<SHIFTED_FORCE, false, HEAT, 0>(s, own, p0, bx, dec0, dec1, dec2, rc2_bits_m1, fshift);
-                    pair_terms<SHIFTED_FORCE, false, HEAT, 0>(s, own, p1, bx, dec0, dec1, dec2, rc2_bits_m1, fshift);
-                    pair_terms<SHIFTED_FORCE, false, HEAT, 0>(s, own, p2, bx, dec0, dec1, dec2, rc2_bits_m1, fshift);
-                    pair_terms<SHIFTED_FORCE, false, HEAT, 0>(s, own, p3, bx, dec0, dec1, dec2, rc2_bits_m1, fshift);
-                }
+                for (const uint4& pj : {p0, p1, p2, p3})
+                    pair_terms<SHIFTED_FORCE, false, HEAT>(s, own, pj, bx, dec0, dec1, dec2, rc2_bits_m1, fshift);
+                if (row & 1u) end_part(s);
             }
         }
-        combine_parts(s);
+        end_part(s);
         if (HEAT) heat_terms(a, bx, i, s, raw);
         disp2 = fmaxf(disp2, advance_slot(a, bx, i, phase, s));
     }
     if (HEAT) block_sum_series(a, raw, sample);
-    block_max_per_box(a, true, 0u, 0u, disp2);
-    if (blockIdx.x == 0 && threadIdx.x == 0) a.glob->pending = 1u;
-    if (!next && !HEAT) return;
-    // the last block to finish takes the next step's rebuild decision and
-    // moves the heat-current series on
-    __shared__ int s_last;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        __threadfence();
-        s_last = atomicAdd(&a.glob->blocks_done, 1u) == gridDim.x - 1u;
-    }
-    __syncthreads();
-    if (!s_last) return;
-    __threadfence();
-    if (threadIdx.x == 0) {
-        a.glob->blocks_done = 0u;
-        if (HEAT) a.glob->heat_next += 1u;
-    }
-    if (next) decide_block(a, next, true, true);
+    finish_step<HEAT>(a, true, 0u, disp2, next);
 }
 
 // ---- measure (lennard_jones.wgsl:576-626) ----
@@ -946,11 +957,11 @@ __global__ void __launch_bounds__(kBlock) begin_kernel(Arena a) {
             a.v[q] = v;
             enc[k] = encode(x, bx.enc[k]);
             const float d = decode_diff(enc[k], sw[k], bx.dec[k]);
-            disp2 += d * d;
+            disp2 = __fmaf_rn(d, d, disp2);
         }
         a.cache[phase ^ 1u][i] = make_uint4(enc[0], enc[1], enc[2], 0u);
     }
-    block_max_per_box(a, valid, b, blockIdx.x * blockDim.x, disp2);
+    note_displacement(a, valid, b, disp2);
     if (i == 0) a.glob->pending = 1u;
 }
 
@@ -1024,7 +1035,7 @@ __device__ __forceinline__ long long warp_sum(long long x) {
 // in which the whole block takes turns on one address (the exchange's pass
 // took 45 us that way at 2,462 atoms, 16.4 us so; Nose-Hoover's 18.5 us at
 // 15,600 atoms, 12.9 us so).
-template <bool SHIFTED_FORCE, int PASS>
+template <bool SHIFTED_FORCE, int PASS, int LANES>
 __global__ void __launch_bounds__(kForceThreads) canon_force_kernel(Arena a,
                                                                     const __grid_constant__ CUtensorMap map) {
     count_kernel(a);
@@ -1032,30 +1043,40 @@ __global__ void __launch_bounds__(kForceThreads) canon_force_kernel(Arena a,
     __shared__ __align__(128) Stage st;
     __shared__ long long s_sum[kWarps][2][9];
     __shared__ int s_last;
-    const uint32_t i = blockIdx.x * kForceThreads + threadIdx.x;
-    const bool valid = i < a.nslots;
+    const uint32_t i = blockIdx.x * (kForceThreads / LANES) + threadIdx.x / LANES;
+    const bool valid = i < a.nslots && threadIdx.x % LANES == 0u;  // lane 0 keeps the particle
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     const Box& bx = a.boxes[0];
-    const PairSums s =
-        block_pair_sums<SHIFTED_FORCE, false>(st, &map, a, bx, i, valid, a.cache[a.glob->phase]);
-    const float acc[3] = {s.ax, s.ay, s.az};
     double v[3] = {0.0, 0.0, 0.0};
     if (valid) {
-        a.acc[i] = make_float4(s.ax, s.ay, s.az, 0.0f);
 #pragma unroll
-        for (int k = 0; k < 3; k++) {
-            const size_t q = (size_t)k * a.seg + i;
-            v[k] = a.v[q];
-            if (PASS != kPrime) {
+        for (int k = 0; k < 3; k++) v[k] = a.v[(size_t)k * a.seg + i];
+    }
+    const int sl = PASS == kExchange && valid ? hex_slab(bx, a.x[2 * (size_t)a.seg + i]) : 2;
+    float acc[3];
+    if constexpr (LANES > 1) {
+        lane_forces<SHIFTED_FORCE, LANES>(a, bx, i, i < a.nslots, threadIdx.x % LANES,
+                                          a.cache[a.glob->phase], acc);
+    } else {
+        const PairSums s =
+            block_pair_sums<SHIFTED_FORCE, false>(st, &map, a, bx, i, valid, a.cache[a.glob->phase]);
+        acc[0] = s.ax;
+        acc[1] = s.ay;
+        acc[2] = s.az;
+    }
+    if (valid) {
+        a.acc[i] = make_float4(acc[0], acc[1], acc[2], 0.0f);
+        if (PASS != kPrime) {
+#pragma unroll
+            for (int k = 0; k < 3; k++) {
                 v[k] += (double)acc[k] * bx.half_dt;
-                a.v[q] = v[k];
+                a.v[(size_t)k * a.seg + i] = v[k];
             }
         }
     }
     if (PASS == kKick) return;
     const double es = (double)bx.energy_scale, ms = (double)bx.momentum_scale;
     if (PASS == kExchange) {
-        const int sl = valid ? hex_slab(bx, a.x[2 * (size_t)a.seg + i]) : 2;
 #pragma unroll
         for (int k = 0; k < 2; k++) {
             const unsigned in = __ballot_sync(0xffffffffu, sl == k);
@@ -1234,14 +1255,6 @@ static void prefer_l1_once() {
     prefer_l1(measure_kernel<false>);
     prefer_l1(prime_kernel<true>);
     prefer_l1(prime_kernel<false>);
-    prefer_l1(canon_force_kernel<true, kPrime>);
-    prefer_l1(canon_force_kernel<false, kPrime>);
-    prefer_l1(canon_force_kernel<true, kNoseHoover>);
-    prefer_l1(canon_force_kernel<false, kNoseHoover>);
-    prefer_l1(canon_force_kernel<true, kExchange>);
-    prefer_l1(canon_force_kernel<false, kExchange>);
-    prefer_l1(canon_force_kernel<true, kKick>);
-    prefer_l1(canon_force_kernel<false, kKick>);
 }
 
 cudaError_t launch_prime(const Arena& a, const CUtensorMap& map, bool shifted_force,
@@ -1252,6 +1265,43 @@ cudaError_t launch_prime(const Arena& a, const CUtensorMap& map, bool shifted_fo
     else
         prime_kernel<false><<<particle_blocks(a), kForceThreads, 0, s>>>(a, map);
     return after_launch();
+}
+
+// Lanes per particle of a force pass over n particles: as many as keep the
+// grid within VLJ_LANE_THREADS_PER_SM threads an SM. There a lane more
+// shortens the chain a warp waits for; past that the warps already cover each
+// other's waits, and the split's shuffles and padded rounds cost more. Pass
+// time inside a graph with 1 / 2 / 4 / 8 lanes (us): 1,000 atoms 8.9 / 13.6 /
+// 7.7 / 6.2; 2,462 (exchange) 15.9 / 12.3 / 10.5 / 9.8; 15,600 (Nose-Hoover)
+// 17.6 / 9.5 / 9.3 / 10.8; 32,768 at rho 0.4 10.1 / 9.4 / 10.0 / 13.1; 64,000
+// 15.2 / 17.8 / 21.7 / 29.6; 256,000 43 / 55 / 71 / 111.
+static int lanes_for(uint32_t n) {
+#ifdef VLJ_LANES_FORCE
+    return VLJ_LANES_FORCE;
+#endif
+    const uint64_t room = (uint64_t)sm_count() * VLJ_LANE_THREADS_PER_SM;
+    for (int lanes = 8; lanes > 1; lanes /= 2)
+        if ((uint64_t)n * (unsigned)lanes <= room) return lanes;
+    return 1;
+}
+
+template <bool SF, int LANES, int THREADS>
+static void launch_lanes(const Arena& a, cudaStream_t s, cudaGraphConditionalHandle next) {
+    static bool carved = false;
+    if (!carved) {
+        carved = true;
+        prefer_l1(step_kernel_lanes<SF, LANES, THREADS>);
+    }
+    step_kernel_lanes<SF, LANES, THREADS>
+        <<<blocks_for(a.nslots, THREADS / LANES), THREADS, 0, s>>>(a, next);
+}
+
+template <bool SF, int THREADS>
+static void launch_step_lanes(const Arena& a, int lanes, cudaStream_t s,
+                              cudaGraphConditionalHandle next) {
+    if (lanes == 8) launch_lanes<SF, 8, THREADS>(a, s, next);
+    else if (lanes == 4) launch_lanes<SF, 4, THREADS>(a, s, next);
+    else launch_lanes<SF, 2, THREADS>(a, s, next);
 }
 
 template <int THREADS>
@@ -1265,24 +1315,15 @@ static cudaError_t launch_step_kernel(const Arena& a, const CUtensorMap& map, bo
         prefer_l1(step_kernel<true, true, THREADS>);
         prefer_l1(step_kernel<false, true, THREADS>);
     }
-    const unsigned blocks = blocks_for(a.nslots, THREADS);
 #if VLJ_LIST_STREAM
-    const bool split = a.step_lanes == 2u ||
-                       (a.step_lanes == 0u && blocks <= (unsigned)sm_count() * kSplitBlocksPerSM);
-    if (!heat && split) {
-        // a grid of a few blocks per SM: two lanes per particle
-        static bool split_carved = false;
-        if (!split_carved) {
-            split_carved = true;
-            prefer_l1(step_kernel_split<true, THREADS>);
-            prefer_l1(step_kernel_split<false, THREADS>);
-        }
-        const unsigned split_blocks = blocks_for(a.nslots, THREADS / 2);
-        if (shifted_force) step_kernel_split<true, THREADS><<<split_blocks, THREADS, 0, s>>>(a, next);
-        else step_kernel_split<false, THREADS><<<split_blocks, THREADS, 0, s>>>(a, next);
+    const int lanes = heat ? 1 : (a.step_lanes ? (int)a.step_lanes : lanes_for(a.nslots));
+    if (lanes > 1) {
+        if (shifted_force) launch_step_lanes<true, THREADS>(a, lanes, s, next);
+        else launch_step_lanes<false, THREADS>(a, lanes, s, next);
         return after_launch();
     }
 #endif
+    const unsigned blocks = blocks_for(a.nslots, THREADS);
     Arena r = a;
 #if VLJ_STEP_REMAP
     static int per_sm = 0;
@@ -1356,18 +1397,37 @@ cudaError_t launch_begin(const Arena& a, cudaStream_t s) {
     return after_launch();
 }
 
+template <bool SF, int PASS, int LANES>
+static void canon_force_lanes(const Arena& a, const CUtensorMap& map, cudaStream_t s) {
+    static bool carved = false;
+    if (!carved) {
+        carved = true;
+        prefer_l1(canon_force_kernel<SF, PASS, LANES>);
+    }
+    canon_force_kernel<SF, PASS, LANES>
+        <<<blocks_for(a.nslots, kForceThreads / LANES), kForceThreads, 0, s>>>(a, map);
+}
+
+template <bool SF, int PASS>
+static void canon_force_pass(const Arena& a, const CUtensorMap& map, cudaStream_t s) {
+#if VLJ_LIST_STREAM
+    switch (lanes_for(a.nslots)) {
+        case 8: return canon_force_lanes<SF, PASS, 8>(a, map, s);
+        case 4: return canon_force_lanes<SF, PASS, 4>(a, map, s);
+        case 2: return canon_force_lanes<SF, PASS, 2>(a, map, s);
+        default: break;
+    }
+#endif
+    canon_force_lanes<SF, PASS, 1>(a, map, s);
+}
+
 template <bool SF>
 static void canon_force(const Arena& a, const CUtensorMap& map, CanonPass pass, cudaStream_t s) {
-    const unsigned blocks = particle_blocks(a);
     switch (pass) {
-        case kPrime: canon_force_kernel<SF, kPrime><<<blocks, kForceThreads, 0, s>>>(a, map); break;
-        case kNoseHoover:
-            canon_force_kernel<SF, kNoseHoover><<<blocks, kForceThreads, 0, s>>>(a, map);
-            break;
-        case kExchange:
-            canon_force_kernel<SF, kExchange><<<blocks, kForceThreads, 0, s>>>(a, map);
-            break;
-        case kKick: canon_force_kernel<SF, kKick><<<blocks, kForceThreads, 0, s>>>(a, map); break;
+        case kPrime: return canon_force_pass<SF, kPrime>(a, map, s);
+        case kNoseHoover: return canon_force_pass<SF, kNoseHoover>(a, map, s);
+        case kExchange: return canon_force_pass<SF, kExchange>(a, map, s);
+        case kKick: return canon_force_pass<SF, kKick>(a, map, s);
     }
 }
 
