@@ -197,11 +197,20 @@ vlj_status upload_particles(vlj_sim* s, const vlj_particle* p, size_t count) {
     return VLJ_OK;
 }
 
+// The rebuild decision, and the rebuild where it is due, ahead of a pass over
+// the lists. Between two such passes with no step (and nothing else that
+// clears lists_current) nothing has moved and the second decision would find
+// nothing to do, so it is not launched.
 vlj_status lists_now(vlj_sim* s) {
+    if (s->lists_current) return VLJ_OK;
     s->one_ready = false;
-    if (s->use_graphs && !s->timing) return sim_launch_lists_graph(s);
-    CUDA_TRY(launch_decide(s->arena, s->stream, 0));
-    CUDA_TRY(launch_rebuild(s->arena, s->stream));
+    if (s->use_graphs && !s->timing) {
+        TRY(sim_launch_lists_graph(s));
+    } else {
+        CUDA_TRY(launch_decide(s->arena, s->stream, 0));
+        CUDA_TRY(launch_rebuild(s->arena, s->stream));
+    }
+    s->lists_current = true;
     return VLJ_OK;
 }
 
@@ -209,6 +218,7 @@ vlj_status lists_now(vlj_sim* s) {
 // velocities into ones half a kick behind (lennard_jones.rs:1080-1089).
 vlj_status restart(vlj_sim* s, const vlj_particle* p, size_t count) {
     s->one_ready = false;
+    s->lists_current = false;
     TRY(upload_particles(s, p, count));
     uint32_t one = 1u;
     CUDA_TRY(cudaMemcpyAsync(&s->arena.ctrl[0].forced, &one, sizeof one, cudaMemcpyHostToDevice,
@@ -263,24 +273,22 @@ vlj_measurement decode(const vlj_sim* s, const Readback& r, uint64_t step) {
     return m;
 }
 
-vlj_status enqueue_measure(vlj_sim* s, bool canonical, int slot) {
+vlj_status enqueue_measure(vlj_sim* s, int slot) {
     CUDA_TRY(cudaMemsetAsync(s->arena.accum, 0, sizeof(unsigned long long) * kSlots, s->stream));
     TRY(lists_now(s));
-    CUDA_TRY(launch_measure(s->arena, s->list_map, s->shifted_force, canonical, s->stream));
+    CUDA_TRY(launch_measure(s->arena, s->list_map, s->shifted_force, s->stream));
     if (s->box.drawn == VLJ_DRAWN_TEMPERATURE) CUDA_TRY(launch_drawn_temperature(s->arena, s->stream));
-    if (slot >= 0) {
-        Readback* r = &s->ring[slot];
-        CUDA_TRY(cudaMemcpyAsync(r->slots, s->arena.accum, sizeof(r->slots), cudaMemcpyDeviceToHost,
+    Readback* r = &s->ring[slot];
+    CUDA_TRY(cudaMemcpyAsync(r->slots, s->arena.accum, sizeof(r->slots), cudaMemcpyDeviceToHost,
+                             s->stream));
+    CUDA_TRY(cudaMemcpyAsync(&r->ctrl, s->arena.ctrl, sizeof(Control), cudaMemcpyDeviceToHost,
+                             s->stream));
+    if (s->nose_hoover)
+        CUDA_TRY(cudaMemcpyAsync(&r->nh, s->arena.nh, sizeof(Thermo), cudaMemcpyDeviceToHost,
                                  s->stream));
-        CUDA_TRY(cudaMemcpyAsync(&r->ctrl, s->arena.ctrl, sizeof(Control), cudaMemcpyDeviceToHost,
-                                 s->stream));
-        if (s->nose_hoover)
-            CUDA_TRY(cudaMemcpyAsync(&r->nh, s->arena.nh, sizeof(Thermo), cudaMemcpyDeviceToHost,
-                                     s->stream));
-        CUDA_TRY(cudaEventRecord(s->ring_event[slot], s->stream));
-        s->ring_busy[slot] = true;
-        s->ring_step[slot] = s->steps;
-    }
+    CUDA_TRY(cudaEventRecord(s->ring_event[slot], s->stream));
+    s->ring_busy[slot] = true;
+    s->ring_step[slot] = s->steps;
     return VLJ_OK;
 }
 
@@ -405,7 +413,7 @@ vlj_status vlj_measure(vlj_sim* s, int* accepted) {
             break;
         }
     if (slot < 0) return VLJ_OK;
-    TRY(enqueue_measure(s, false, slot));
+    TRY(enqueue_measure(s, slot));
     *accepted = 1;
     return VLJ_OK;
 }
@@ -458,8 +466,9 @@ vlj_status vlj_measure_now(vlj_sim* s, vlj_measurement* out) {
 
 vlj_status vlj_read_particles(vlj_sim* s, vlj_particle* out) {
     if (!s || !out) return fail(VLJ_INVALID_ARG, "null argument");
-    TRY(enqueue_measure(s, true, -1));
-    CUDA_TRY(launch_store_particles(s->arena, s->stream));
+    TRY(lists_now(s));
+    CUDA_TRY(launch_read(s->arena, s->list_map, s->shifted_force, 0, s->n, s->arena.aos, s->stream));
+    if (s->box.drawn == VLJ_DRAWN_TEMPERATURE) CUDA_TRY(launch_drawn_temperature(s->arena, s->stream));
     CUDA_TRY(cudaMemcpyAsync(out, s->arena.aos, sizeof(vlj_particle) * s->n, cudaMemcpyDeviceToHost,
                              s->stream));
     CUDA_TRY(cudaStreamSynchronize(s->stream));
@@ -698,6 +707,7 @@ vlj_status vlj_debug_force_rebuild(vlj_sim* s) {
     uint32_t one = 1u;
     CUDA_TRY(cudaMemcpyAsync(&s->arena.ctrl[0].forced, &one, sizeof one, cudaMemcpyHostToDevice,
                              s->stream));
+    s->lists_current = false;
     TRY(lists_now(s));
     CUDA_TRY(cudaStreamSynchronize(s->stream));
     return VLJ_OK;
@@ -1144,7 +1154,6 @@ vlj_status sim_allocate(vlj_sim* s, void* stream) {
     TRY(dalloc(s, &a.pe_half, 2 * (size_t)seg));
     TRY(dalloc(s, &a.w_half, 2 * (size_t)seg));
     TRY(dalloc(s, &a.vel4, seg));
-    TRY(dalloc(s, &a.vcanon, 3 * (size_t)seg));
     if (!batched && s->box.profile_bins)
         TRY(dalloc(s, &a.profile, (size_t)s->box.profile_bins * 8 + 3));
     // the last cell of the last box ends at the last slot
@@ -1338,6 +1347,7 @@ static vlj_status step_direct(vlj_sim* s, bool heat = false) {
 }
 
 vlj_status sim_enqueue_steps(vlj_sim* s, uint32_t steps) {
+    if (steps > 0) s->lists_current = false;
     if (steps > 0 && s->heat_pending) {
         // the first step's force pass takes the requested heat-current sample
         if (s->timing || !s->use_graphs) {
@@ -1467,6 +1477,7 @@ vlj_status sim_grow_lists(vlj_sim* s, bool* grew) {
     s->list_grows += 1;
     *grew = true;
     // the forced rebuild now, so what follows reads full lists
+    s->lists_current = false;
     return lists_now(s);
 }
 

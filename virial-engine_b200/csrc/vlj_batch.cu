@@ -113,15 +113,15 @@ vlj_measurement decode(const vlj_sim* s, const Box& bx, const long long* slots,
     return m;
 }
 
-// Forces, energies and canonical velocities of every box now (the lists
-// brought up to date first); the sums land in a.accum.
-vlj_status measure_all(vlj_batch* bt, bool canonical) {
+// Energies and sums of every box now (the lists brought up to date first);
+// they land in a.accum.
+vlj_status measure_all(vlj_batch* bt) {
     vlj_sim* s = bt->sim;
     const size_t boxes = s->replicas.size();
     CUDA_TRY(cudaMemsetAsync(s->arena.accum, 0, sizeof(unsigned long long) * kSlots * boxes,
                              s->stream));
     TRY(sim_lists_now(s));
-    CUDA_TRY(launch_measure(s->arena, s->list_map, s->shifted_force, canonical, s->stream));
+    CUDA_TRY(launch_measure(s->arena, s->list_map, s->shifted_force, s->stream));
     return VLJ_OK;
 }
 
@@ -240,7 +240,7 @@ vlj_status vlj_batch_measure(vlj_batch* bt, vlj_measurement* out) {
     if (!bt || !out) return fail(VLJ_INVALID_ARG, "null argument");
     vlj_sim* s = bt->sim;
     const size_t boxes = s->replicas.size();
-    TRY(measure_all(bt, false));
+    TRY(measure_all(bt));
     CUDA_TRY(cudaMemcpyAsync(bt->accum, s->arena.accum, sizeof(long long) * kSlots * boxes,
                              cudaMemcpyDeviceToHost, s->stream));
     CUDA_TRY(cudaMemcpyAsync(bt->ctrl, s->arena.ctrl, sizeof(Control) * boxes,
@@ -266,26 +266,12 @@ vlj_status vlj_batch_read_particles(vlj_batch* bt, size_t replica, vlj_particle*
     if (replica >= s->replicas.size())
         return fail(VLJ_INVALID_ARG, "replica %zu of %zu", replica, s->replicas.size());
     const Box& bx = s->replicas[replica];
-    const size_t seg = s->arena.seg, first = bx.first, n = bx.n;
-    TRY(measure_all(bt, true));
-    for (int k = 0; k < 3; k++) {
-        CUDA_TRY(cudaMemcpyAsync(s->pin_x + k * seg + first, s->arena.x + k * seg + first,
-                                 sizeof(double) * n, cudaMemcpyDeviceToHost, s->stream));
-        CUDA_TRY(cudaMemcpyAsync(s->pin_v + k * seg + first, s->arena.vcanon + k * seg + first,
-                                 sizeof(double) * n, cudaMemcpyDeviceToHost, s->stream));
-    }
-    CUDA_TRY(cudaMemcpyAsync(s->pin_id + first, s->arena.id + first, sizeof(uint32_t) * n,
-                             cudaMemcpyDeviceToHost, s->stream));
-    CUDA_TRY(cudaStreamSynchronize(s->stream));
+    // this replica's particles alone, already in input order
+    TRY(sim_lists_now(s));
+    CUDA_TRY(launch_read(s->arena, s->list_map, s->shifted_force, bx.first, bx.n, s->arena.aos, s->stream));
+    CUDA_TRY(cudaMemcpyAsync(out, s->arena.aos, sizeof(vlj_particle) * bx.n, cudaMemcpyDeviceToHost,
+                             s->stream));
     TRY(check_fault(s));
-    for (size_t slot = first; slot < first + n; slot++) {
-        const uint32_t i = s->pin_id[slot];
-        if (i >= n) return fail(VLJ_CUDA_ERROR, "corrupt particle id %u in slot %zu", i, slot);
-        for (int k = 0; k < 3; k++) {
-            out[i].pos[k] = s->pin_x[k * seg + slot];
-            out[i].vel[k] = s->pin_v[k * seg + slot];
-        }
-    }
     return VLJ_OK;
 }
 

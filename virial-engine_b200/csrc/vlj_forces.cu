@@ -46,6 +46,8 @@ struct PairSums {
     // az) in list order (end_part). One thread walking all rows and several
     // lanes taking a part each then give the same bits.
     float px, py, pz;
+    // likewise the part's energies and virials
+    float ppe, ppe_lo, pw, pw_lo;
 };
 
 __device__ __forceinline__ void end_part(PairSums& s) {
@@ -53,6 +55,35 @@ __device__ __forceinline__ void end_part(PairSums& s) {
     s.ay = __fadd_rn(s.ay, s.py);
     s.az = __fadd_rn(s.az, s.pz);
     s.px = s.py = s.pz = 0.0f;
+}
+
+// A part's energy and virial into the totals, hi and lo.
+__device__ __forceinline__ void add_part_energies(PairSums& s, float pe, float pe_lo, float w,
+                                                  float w_lo) {
+    float t, e;
+    two_sum(s.pe, pe, t, e);
+    s.pe = t;
+    s.pe_lo = __fadd_rn(s.pe_lo, __fadd_rn(pe_lo, e));
+    two_sum(s.w, w, t, e);
+    s.w = t;
+    s.w_lo = __fadd_rn(s.w_lo, __fadd_rn(w_lo, e));
+}
+
+// end_part with the energies.
+template <bool ENERGIES>
+__device__ __forceinline__ void finish_part(PairSums& s) {
+    end_part(s);
+    if (ENERGIES) {
+        add_part_energies(s, s.ppe, s.ppe_lo, s.pw, s.pw_lo);
+        s.ppe = s.ppe_lo = s.pw = s.pw_lo = 0.0f;
+    }
+}
+
+// A 32-bit integer as f64, exactly, by its bits in the fraction of 2^52 +
+// 2^31: an f64 subtraction in place of the conversion, whose unit takes a
+// quarter of the FP64 pipe's rate.
+__device__ __forceinline__ double int_to_double(uint32_t x) {
+    return __dsub_rn(__hiloint2double(0x43300000, (int)(x ^ 0x80000000u)), 4503601774854144.0);
 }
 
 __device__ __forceinline__ void add_force(PairSums& s, float dx, float dy, float dz, float f) {
@@ -143,7 +174,7 @@ __device__ __forceinline__ bool bar_wait(unsigned long long* bar, uint32_t parit
 // the halves of the pair energy and virial as unevaluated f32 pairs (as the
 // reference sums them in double-float, lennard_jones.wgsl:518-519). A zero
 // separation (the padding of a list's last row) adds nothing.
-template <bool SHIFTED_FORCE, bool ENERGIES, bool HEAT>
+template <bool SHIFTED_FORCE, bool ENERGIES, bool HEAT, bool NEAR = false>
 __device__ __forceinline__ void pair_terms(PairSums& s, const uint4 own, const uint4 pj,
                                            const Box& bx, float dec0, float dec1, float dec2,
                                            uint32_t rc2_bits_m1, float fshift) {
@@ -171,19 +202,19 @@ __device__ __forceinline__ void pair_terms(PairSums& s, const uint4 own, const u
         // integer differences times the box step are exact in f64): on a
         // lattice, where every pair at one distance rounds alike, the f32
         // components' three roundings would bias the virial coherently.
-        const double ex = (double)(int32_t)(pj.x - own.x) * (double)dec0;
-        const double ey = (double)(int32_t)(pj.y - own.y) * (double)dec1;
-        const double ez = (double)(int32_t)(pj.z - own.z) * (double)dec2;
+        const double ex = int_to_double(pj.x - own.x) * (double)dec0;
+        const double ey = int_to_double(pj.y - own.y) * (double)dec1;
+        const double ez = int_to_double(pj.z - own.z) * (double)dec2;
         float rf, u, t, e;
-        lj_pair<SHIFTED_FORCE>((float)(ex * ex + ey * ey + ez * ez), bx, rf, u);
-        two_sum(s.pe, 0.5f * u, t, e);
-        s.pe = t;
-        s.pe_lo += e;
-        two_sum(s.w, 0.5f * rf, t, e);
-        s.w = t;
-        s.w_lo += e;
-        s.near += r2 < 2.25f ? 1u : 0u;
+        lj_pair<SHIFTED_FORCE>((float)__fma_rn(ez, ez, __fma_rn(ey, ey, __dmul_rn(ex, ex))), bx, rf, u);
+        two_sum(s.ppe, 0.5f * u, t, e);
+        s.ppe = t;
+        s.ppe_lo += e;
+        two_sum(s.pw, 0.5f * rf, t, e);
+        s.pw = t;
+        s.pw_lo += e;
     }
+    if (ENERGIES || NEAR) s.near += in && r2 < 2.25f ? 1u : 0u;
 }
 
 // pair_terms on positions given as f32 offsets from a common origin near
@@ -212,15 +243,15 @@ __device__ __forceinline__ void pair_terms_rel(PairSums& s, const float4 own, co
 
 // The particle's pair sums over its list. Every thread of the block must
 // call this: it synchronises the block between tiles.
-template <bool SHIFTED_FORCE, bool ENERGIES, bool HEAT = false>
+template <bool SHIFTED_FORCE, bool ENERGIES, bool HEAT = false, bool NEAR = false>
 __device__ __forceinline__ PairSums block_pair_sums(Stage& st, const CUtensorMap* map,
                                                     const Arena& a, const Box& bx, uint32_t i,
-                                                    bool valid, const uint4* __restrict__ cur) {
-    PairSums s = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0u,
-                  0.0f, {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f}};
+                                                    bool valid, const uint4* __restrict__ cur,
+                                                    uint32_t block0 = 0) {
+    PairSums s = {};
 #if !VLJ_LIST_STREAM
-    const uint32_t first = blockIdx.x * kForceThreads;
-    const uint32_t rows = a.block_rows[blockIdx.x];
+    const uint32_t first = (block0 + blockIdx.x) * kForceThreads;
+    const uint32_t rows = a.block_rows[block0 + blockIdx.x];
     const uint32_t tiles = (rows + kTileRows - 1u) / kTileRows;
     if (threadIdx.x == 0) {
         for (int k = 0; k < kTileSlots; k++) bar_init(&st.bar[k]);
@@ -233,6 +264,7 @@ __device__ __forceinline__ PairSums block_pair_sums(Stage& st, const CUtensorMap
 #else
     (void)st;
     (void)map;
+    (void)block0;  // the grid's first block of kForceThreads slots (the TMA tiles' unit)
 #endif
 
     uint4 own = make_uint4(0u, 0u, 0u, 0u);
@@ -249,8 +281,8 @@ __device__ __forceinline__ PairSums block_pair_sums(Stage& st, const CUtensorMap
     // The list's last row is padded with the particle itself, whose zero
     // separation drops out with the entries beyond the cutoff.
     auto add = [&](const uint4 pj) {
-        pair_terms<SHIFTED_FORCE, ENERGIES, HEAT>(s, own, pj, bx, dec0, dec1, dec2,
-                                                  rc2_bits_m1, fshift);
+        pair_terms<SHIFTED_FORCE, ENERGIES, HEAT, NEAR>(s, own, pj, bx, dec0, dec1, dec2,
+                                                        rc2_bits_m1, fshift);
     };
     // the four entries of list row `row`; a part ends with its odd row
     auto row_terms = [&](uint32_t row, const uint4 p0, const uint4 p1, const uint4 p2,
@@ -259,7 +291,7 @@ __device__ __forceinline__ PairSums block_pair_sums(Stage& st, const CUtensorMap
         add(p1);
         add(p2);
         add(p3);
-        if (row & 1u) end_part(s);
+        if (row & 1u) finish_part<ENERGIES>(s);
     };
 
 #if VLJ_LIST_STREAM
@@ -317,11 +349,11 @@ __device__ __forceinline__ PairSums block_pair_sums(Stage& st, const CUtensorMap
             add(p1);
             add(p2);
             add(p3);
-            end_part(s);
+            finish_part<ENERGIES>(s);
         }
     }
 #endif
-    end_part(s);
+    finish_part<ENERGIES>(s);
     return s;
 #else
     bool lost = false;
@@ -362,22 +394,22 @@ __device__ __forceinline__ PairSums block_pair_sums(Stage& st, const CUtensorMap
         }
         __syncthreads();
     }
-    end_part(s);
+    finish_part<ENERGIES>(s);
     return s;
 #endif
 }
 
-// The force on particle i (all components in every lane) with LANES
-// consecutive threads sharing its list: in each round lane `sub` sums part
-// round * LANES + sub (two rows, eight gathers in flight), and the round's
-// parts join the total in list order, so the bits are block_pair_sums's. The
-// next round's rows load behind this one's pairs. A row past the list's end
-// reads as the particle itself, whose zero separation adds nothing. Every
-// lane of the warp must call this.
-template <bool SHIFTED_FORCE, int LANES>
-__device__ __forceinline__ void lane_forces(const Arena& a, const Box& bx, uint32_t i, bool valid,
-                                            uint32_t sub, const uint4* __restrict__ cur,
-                                            float (&f)[3]) {
+// The pair sums of particle i (in every lane) with LANES consecutive threads
+// sharing its list: in each round lane `sub` sums part round * LANES + sub
+// (two rows, eight gathers in flight), and the round's parts join the totals
+// in list order, so the bits are block_pair_sums's. The next round's rows load
+// behind this one's pairs. A row past the list's end reads as the particle
+// itself, whose zero separation adds nothing. Every lane of the warp must call
+// this.
+template <bool SHIFTED_FORCE, int LANES, bool ENERGIES = false, bool NEAR = false>
+__device__ __forceinline__ PairSums lane_pair_sums(const Arena& a, const Box& bx, uint32_t i,
+                                                   bool valid, uint32_t sub,
+                                                   const uint4* __restrict__ cur) {
     const uint32_t at = valid ? i : 0u;
     const uint4 own = __ldg(cur + at);
     const uint32_t rows = valid ? (__ldg(a.list_count + at) + 3u) / 4u : 0u;
@@ -391,26 +423,36 @@ __device__ __forceinline__ void lane_forces(const Arena& a, const Box& bx, uint3
     uint32_t row = 2u * sub;
     uint4 e0 = row < rows ? load_row_streaming(rowp + (size_t)row * a.seg) : self;
     uint4 e1 = row + 1u < rows ? load_row_streaming(rowp + (size_t)(row + 1u) * a.seg) : self;
-    f[0] = f[1] = f[2] = 0.0f;
+    PairSums s = {};
     for (uint32_t r = 0; r < rounds; r++) {
         const uint4 p[8] = {__ldg(cur + e0.x), __ldg(cur + e0.y), __ldg(cur + e0.z), __ldg(cur + e0.w),
                             __ldg(cur + e1.x), __ldg(cur + e1.y), __ldg(cur + e1.z), __ldg(cur + e1.w)};
         row += 2u * LANES;
         e0 = row < rows ? load_row_streaming(rowp + (size_t)row * a.seg) : self;
         e1 = row + 1u < rows ? load_row_streaming(rowp + (size_t)(row + 1u) * a.seg) : self;
-        PairSums s = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0u,
-                      0.0f, {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f}};
+        s.px = s.py = s.pz = 0.0f;
+        s.ppe = s.ppe_lo = s.pw = s.pw_lo = 0.0f;
 #pragma unroll
         for (int k = 0; k < 8; k++)
-            pair_terms<SHIFTED_FORCE, false, false>(s, own, p[k], bx, dec0, dec1, dec2, rc2_bits_m1,
-                                                    fshift);
+            pair_terms<SHIFTED_FORCE, ENERGIES, false, NEAR>(s, own, p[k], bx, dec0, dec1, dec2,
+                                                             rc2_bits_m1, fshift);
 #pragma unroll
         for (int k = 0; k < LANES; k++) {
-            f[0] = __fadd_rn(f[0], __shfl_sync(0xffffffffu, s.px, k, LANES));
-            f[1] = __fadd_rn(f[1], __shfl_sync(0xffffffffu, s.py, k, LANES));
-            f[2] = __fadd_rn(f[2], __shfl_sync(0xffffffffu, s.pz, k, LANES));
+            s.ax = __fadd_rn(s.ax, __shfl_sync(0xffffffffu, s.px, k, LANES));
+            s.ay = __fadd_rn(s.ay, __shfl_sync(0xffffffffu, s.py, k, LANES));
+            s.az = __fadd_rn(s.az, __shfl_sync(0xffffffffu, s.pz, k, LANES));
+            if (ENERGIES)
+                add_part_energies(s, __shfl_sync(0xffffffffu, s.ppe, k, LANES),
+                                  __shfl_sync(0xffffffffu, s.ppe_lo, k, LANES),
+                                  __shfl_sync(0xffffffffu, s.pw, k, LANES),
+                                  __shfl_sync(0xffffffffu, s.pw_lo, k, LANES));
         }
     }
+    if (ENERGIES || NEAR) {
+#pragma unroll
+        for (int o = 1; o < LANES; o <<= 1) s.near += __shfl_xor_sync(0xffffffffu, s.near, o);
+    }
+    return s;
 }
 
 // Sum of one heat-current sample's three components over the block into
@@ -642,7 +684,7 @@ __global__ void __launch_bounds__(THREADS, kStepMinBlocks) step_kernel(Arena a,
 // ---- one step with LANES lanes per particle, for grids that leave the chip
 // idle at one (lanes_for): a lone warp cannot hide its latency behind others,
 // so its chain of rows and gathers is what the step takes. The list's parts
-// go to the lanes (lane_forces); with four lanes or more, lane c < 3 then
+// go to the lanes (lane_pair_sums); with four lanes or more, lane c < 3 then
 // steps component c, its state loaded before the forces. The same step as
 // step_kernel to the bit (no heat-current sample). ----
 template <bool SHIFTED_FORCE, int LANES, int THREADS>
@@ -655,7 +697,6 @@ __global__ void __launch_bounds__(THREADS) step_kernel_lanes(Arena a, cudaGraphC
     const uint32_t phase = a.glob->phase;
     const uint32_t b = valid ? box_of_slot(a, i) : 0u;
     const Box& bx = a.boxes[b];
-    float f[3];
     if constexpr (LANES >= 4) {
         const bool mine = valid && sub < 3u;
         const size_t q = (size_t)sub * a.seg + i;
@@ -667,11 +708,11 @@ __global__ void __launch_bounds__(THREADS) step_kernel_lanes(Arena a, cudaGraphC
             sw = reinterpret_cast<const uint32_t*>(a.snap + i)[sub];
             if (bx.thermostat == 1) id = a.id[i];
         }
-        lane_forces<SHIFTED_FORCE, LANES>(a, bx, i, valid, sub, a.cache[phase], f);
+        const PairSums s = lane_pair_sums<SHIFTED_FORCE, LANES>(a, bx, i, valid, sub, a.cache[phase]);
         float d = 0.0f;
         if (mine) {
             const float xi = bx.thermostat == 1 ? langevin_noise_of(sub, id, a.glob->step, bx.seed) : 0.0f;
-            advance_component(bx, bx.box[sub], sub == 0u ? f[0] : (sub == 1u ? f[1] : f[2]), xi, x, v);
+            advance_component(bx, bx.box[sub], sub == 0u ? s.ax : (sub == 1u ? s.ay : s.az), xi, x, v);
             a.x[q] = x;
             a.v[q] = v;
             const uint32_t enc = encode(x, bx.enc[sub]);
@@ -686,8 +727,7 @@ __global__ void __launch_bounds__(THREADS) step_kernel_lanes(Arena a, cudaGraphC
         }
         finish_step<false>(a, valid, b, disp2, next);
     } else {
-        lane_forces<SHIFTED_FORCE, LANES>(a, bx, i, valid, sub, a.cache[phase], f);
-        const PairSums s = {f[0], f[1], f[2]};
+        const PairSums s = lane_pair_sums<SHIFTED_FORCE, LANES>(a, bx, i, valid, sub, a.cache[phase]);
         const bool mine = valid && sub == 0u;
         finish_step<false>(a, mine, b, mine ? advance_slot(a, bx, i, phase, s) : 0.0f, next);
     }
@@ -778,8 +818,7 @@ __global__ void __launch_bounds__(kBlock) tile_step_kernel(Arena a, cudaGraphCon
     for (uint32_t p = h0 + threadIdx.x; p < h1; p += blockDim.x) {
         const uint32_t i = a.sorted[p];
         const uint32_t cnt = a.list_count[i];
-        PairSums s = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0u,
-                      0.0f, {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f}};
+        PairSums s = {};
         if (staged) {
 #if VLJ_TILE_F32
             const float4 own = s_tilef[own0 + p];
@@ -870,18 +909,23 @@ __global__ void __launch_bounds__(kBlock) tile_step_kernel(Arena a, cudaGraphCon
 // 1.5 sigma, the velocity at the step (stored velocity plus the closing half
 // kick), kinetic energy and momentum in f64. Each value goes to 32.32 fixed
 // point scaled like the reference and is summed exactly.
-template <bool SHIFTED_FORCE>
+// Several lanes per particle on small grids, as in the step (lanes_for).
+template <bool SHIFTED_FORCE, int LANES>
 __global__ void __launch_bounds__(kForceThreads) measure_kernel(Arena a,
-                                                                const __grid_constant__ CUtensorMap map,
-                                                                int canonical) {
+                                                                const __grid_constant__ CUtensorMap map) {
     count_kernel(a);
     __shared__ __align__(128) Stage st;
-    const uint32_t i = blockIdx.x * kForceThreads + threadIdx.x;
-    const bool valid = i < a.nslots;
-    const uint32_t b = valid ? box_of_slot(a, i) : 0u;
+    constexpr uint32_t kPer = kForceThreads / LANES;
+    const uint32_t i = blockIdx.x * kPer + threadIdx.x / LANES;
+    const uint32_t b = i < a.nslots ? box_of_slot(a, i) : 0u;
     const Box& bx = a.boxes[b];
-    const PairSums s =
-        block_pair_sums<SHIFTED_FORCE, true>(st, &map, a, bx, i, valid, a.cache[a.glob->phase]);
+    const bool valid = i < a.nslots && threadIdx.x % LANES == 0u;  // lane 0 keeps the particle
+    PairSums s;
+    if constexpr (LANES > 1)
+        s = lane_pair_sums<SHIFTED_FORCE, LANES, true>(a, bx, i, i < a.nslots, threadIdx.x % LANES,
+                                                       a.cache[a.glob->phase]);
+    else
+        s = block_pair_sums<SHIFTED_FORCE, true>(st, &map, a, bx, i, valid, a.cache[a.glob->phase]);
     long long v[kSlots] = {0, 0, 0, 0, 0, 0, 0, 0};
     if (valid) {
         const float acc[3] = {s.ax, s.ay, s.az};
@@ -890,7 +934,6 @@ __global__ void __launch_bounds__(kForceThreads) measure_kernel(Arena a,
         for (int k = 0; k < 3; k++) {
             vel[k] = canonical_velocity(a, bx, b, i, k, acc[k]);
             ke += vel[k] * vel[k];
-            if (canonical) a.vcanon[(size_t)k * a.seg + i] = vel[k];
         }
         ke *= 0.5;
         const double es = (double)bx.energy_scale, ms = (double)bx.momentum_scale;
@@ -906,7 +949,48 @@ __global__ void __launch_bounds__(kForceThreads) measure_kernel(Arena a,
         a.w_half[2 * i + 1] = s.w_lo;
         a.vel4[i] = make_float4((float)vel[0], (float)vel[1], (float)vel[2], (float)s.near);
     }
-    block_sum_slots(a, valid, b, blockIdx.x * kForceThreads, v);
+    block_sum_slots(a, valid, b, blockIdx.x * kPer, v);
+}
+
+// ---- particles out (lennard_jones.rs:1354-1374; input order) ----
+// Slots first .. first + count - 1 (one box, or a replica's): the forces for
+// the canonical velocity and the neighbours within 1.5 sigma, with no
+// energies, then positions and velocities straight into the particles as the
+// API passes them, at out[id]. A measurement in its place computed every
+// pair's energy in f64 for nothing (95 us at 256,000 atoms, 42 us so).
+template <bool SHIFTED_FORCE, int LANES>
+__global__ void __launch_bounds__(kForceThreads) read_kernel(Arena a, const __grid_constant__ CUtensorMap map,
+                                                             uint32_t first, uint32_t count,
+                                                             double* __restrict__ out) {
+    count_kernel(a);
+    __shared__ __align__(128) Stage st;
+    const uint32_t sub = threadIdx.x % LANES;
+    // the grid starts at the slot of its first whole block
+    const uint32_t block0 = LANES == 1 ? first / kForceThreads : 0u;
+    const uint32_t from = LANES == 1 ? block0 * kForceThreads : first;
+    const uint32_t i = from + blockIdx.x * (kForceThreads / LANES) + threadIdx.x / LANES;
+    const bool valid = i >= first && i - first < count;
+    const uint32_t b = valid ? box_of_slot(a, i) : 0u;
+    const Box& bx = a.boxes[b];
+    PairSums s;
+    if constexpr (LANES > 1)
+        s = lane_pair_sums<SHIFTED_FORCE, LANES, false, true>(a, bx, i, valid, sub, a.cache[a.glob->phase]);
+    else
+        s = block_pair_sums<SHIFTED_FORCE, false, false, true>(st, &map, a, bx, i, valid,
+                                                               a.cache[a.glob->phase], block0);
+    if (!valid || sub != 0u) return;
+    const double v[3] = {canonical_velocity(a, bx, b, i, 0, s.ax), canonical_velocity(a, bx, b, i, 1, s.ay),
+                         canonical_velocity(a, bx, b, i, 2, s.az)};
+    a.vel4[i] = make_float4((float)v[0], (float)v[1], (float)v[2], (float)s.near);
+    const uint32_t id = a.id[i];
+    if (id >= count) {
+        atomicCAS(&a.glob->fault, 0u, kFaultBadId);
+        return;
+    }
+    double2* p = reinterpret_cast<double2*>(out) + 3 * (size_t)id;
+    p[0] = make_double2(a.x[i], a.x[(size_t)a.seg + i]);
+    p[1] = make_double2(a.x[2 * (size_t)a.seg + i], v[0]);
+    p[2] = make_double2(v[1], v[2]);
 }
 
 // ---- steps on canonical velocities: Nose-Hoover (lennard_jones.wgsl:309-397)
@@ -1053,17 +1137,13 @@ __global__ void __launch_bounds__(kForceThreads) canon_force_kernel(Arena a,
         for (int k = 0; k < 3; k++) v[k] = a.v[(size_t)k * a.seg + i];
     }
     const int sl = PASS == kExchange && valid ? hex_slab(bx, a.x[2 * (size_t)a.seg + i]) : 2;
-    float acc[3];
-    if constexpr (LANES > 1) {
-        lane_forces<SHIFTED_FORCE, LANES>(a, bx, i, i < a.nslots, threadIdx.x % LANES,
-                                          a.cache[a.glob->phase], acc);
-    } else {
-        const PairSums s =
-            block_pair_sums<SHIFTED_FORCE, false>(st, &map, a, bx, i, valid, a.cache[a.glob->phase]);
-        acc[0] = s.ax;
-        acc[1] = s.ay;
-        acc[2] = s.az;
-    }
+    PairSums s;
+    if constexpr (LANES > 1)
+        s = lane_pair_sums<SHIFTED_FORCE, LANES>(a, bx, i, i < a.nslots, threadIdx.x % LANES,
+                                                 a.cache[a.glob->phase]);
+    else
+        s = block_pair_sums<SHIFTED_FORCE, false>(st, &map, a, bx, i, valid, a.cache[a.glob->phase]);
+    const float acc[3] = {s.ax, s.ay, s.az};
     if (valid) {
         a.acc[i] = make_float4(acc[0], acc[1], acc[2], 0.0f);
         if (PASS != kPrime) {
@@ -1251,8 +1331,6 @@ static void prefer_l1_once() {
     static bool done = false;
     if (done) return;
     done = true;
-    prefer_l1(measure_kernel<true>);
-    prefer_l1(measure_kernel<false>);
     prefer_l1(prime_kernel<true>);
     prefer_l1(prime_kernel<false>);
 }
@@ -1382,13 +1460,66 @@ cudaError_t launch_step(const Arena& a, const CUtensorMap& map, bool shifted_for
 #endif
 }
 
-cudaError_t launch_measure(const Arena& a, const CUtensorMap& map, bool shifted_force,
-                           bool canonical, cudaStream_t s) {
-    prefer_l1_once();
-    if (shifted_force)
-        measure_kernel<true><<<particle_blocks(a), kForceThreads, 0, s>>>(a, map, canonical ? 1 : 0);
-    else
-        measure_kernel<false><<<particle_blocks(a), kForceThreads, 0, s>>>(a, map, canonical ? 1 : 0);
+template <bool SF, int LANES>
+static void measure_lanes(const Arena& a, const CUtensorMap& map, cudaStream_t s) {
+    static bool carved = false;
+    if (!carved) {
+        carved = true;
+        prefer_l1(measure_kernel<SF, LANES>);
+    }
+    measure_kernel<SF, LANES><<<blocks_for(a.nslots, kForceThreads / LANES), kForceThreads, 0, s>>>(a, map);
+}
+
+template <bool SF>
+static void measure(const Arena& a, const CUtensorMap& map, cudaStream_t s) {
+#if VLJ_LIST_STREAM
+    switch (lanes_for(a.nslots)) {
+        case 8: return measure_lanes<SF, 8>(a, map, s);
+        case 4: return measure_lanes<SF, 4>(a, map, s);
+        case 2: return measure_lanes<SF, 2>(a, map, s);
+        default: break;
+    }
+#endif
+    measure_lanes<SF, 1>(a, map, s);
+}
+
+cudaError_t launch_measure(const Arena& a, const CUtensorMap& map, bool shifted_force, cudaStream_t s) {
+    if (shifted_force) measure<true>(a, map, s);
+    else measure<false>(a, map, s);
+    return after_launch();
+}
+
+template <bool SF, int LANES>
+static void read_lanes(const Arena& a, const CUtensorMap& map, uint32_t first, uint32_t count, double* out,
+                       cudaStream_t s) {
+    static bool carved = false;
+    if (!carved) {
+        carved = true;
+        prefer_l1(read_kernel<SF, LANES>);
+    }
+    const uint32_t before = LANES == 1 ? first % kForceThreads : 0u;
+    read_kernel<SF, LANES><<<blocks_for((uint64_t)before + count, kForceThreads / LANES), kForceThreads, 0, s>>>(
+        a, map, first, count, out);
+}
+
+template <bool SF>
+static void read(const Arena& a, const CUtensorMap& map, uint32_t first, uint32_t count, double* out,
+                 cudaStream_t s) {
+#if VLJ_LIST_STREAM
+    switch (lanes_for(count)) {
+        case 8: return read_lanes<SF, 8>(a, map, first, count, out, s);
+        case 4: return read_lanes<SF, 4>(a, map, first, count, out, s);
+        case 2: return read_lanes<SF, 2>(a, map, first, count, out, s);
+        default: break;
+    }
+#endif
+    read_lanes<SF, 1>(a, map, first, count, out, s);
+}
+
+cudaError_t launch_read(const Arena& a, const CUtensorMap& map, bool shifted_force, uint32_t first,
+                        uint32_t count, double* out, cudaStream_t s) {
+    if (shifted_force) read<true>(a, map, first, count, out, s);
+    else read<false>(a, map, first, count, out, s);
     return after_launch();
 }
 

@@ -50,7 +50,7 @@ __global__ void encode_kernel(Arena a) {
     a.cache[a.glob->phase][i] = w;
 }
 
-// ---- particles in and out (lennard_jones.rs:1354-1374; input order) ----
+// ---- particles in (lennard_jones.rs:1354-1374; input order) ----
 __global__ void load_particles_kernel(Arena a) {
     count_kernel(a);
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -70,18 +70,6 @@ __global__ void load_particles_kernel(Arena a) {
     }
     a.id[i] = i;
     if (!finite) atomicCAS(&a.glob->fault, 0u, kFaultNonFinite);
-}
-
-__global__ void store_particles_kernel(Arena a) {
-    count_kernel(a);
-    const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= a.nslots) return;
-    double* p = a.aos + 6 * (size_t)a.id[s];
-#pragma unroll
-    for (int k = 0; k < 3; k++) {
-        p[k] = a.x[(size_t)k * a.seg + s];
-        p[3 + k] = a.vcanon[(size_t)k * a.seg + s];
-    }
 }
 
 // ---- decide (lennard_jones.wgsl:281-307) ----
@@ -452,11 +440,6 @@ cudaError_t launch_encode(const Arena& a, cudaStream_t s) {
 
 cudaError_t launch_load_particles(const Arena& a, cudaStream_t s) {
     load_particles_kernel<<<blocks_for(a.nslots), kBlock, 0, s>>>(a);
-    return after_launch();
-}
-
-cudaError_t launch_store_particles(const Arena& a, cudaStream_t s) {
-    store_particles_kernel<<<blocks_for(a.nslots), kBlock, 0, s>>>(a);
     return after_launch();
 }
 

@@ -209,6 +209,7 @@ struct Exchange {
 // Fault codes in Global::fault (the first one recorded wins).
 constexpr uint32_t kFaultTmaTimeout = 1;  // a TMA tile never arrived
 constexpr uint32_t kFaultNonFinite = 2;   // an uploaded coordinate was not finite
+constexpr uint32_t kFaultBadId = 3;       // a particle's id was not one of its box's
 
 // Every pointer a kernel needs; passed by value (it sits in the constant
 // bank), so captured graphs see fixed pointers and read the mutable state
@@ -282,7 +283,6 @@ struct Arena {
     float* pe_half;  // (hi, lo) per slot
     float* w_half;   // (hi, lo) per slot
     float4* vel4;
-    double* vcanon;             // canonical velocities (3 * seg), on request
     // profiles / heat current
     unsigned long long* profile;  // bins * 8 + 3 per box
     unsigned long long* series;   // 1 + 3 * capacity
@@ -471,10 +471,8 @@ __device__ __forceinline__ float encoded_r2(uint4 a, uint4 b, const float dec[3]
 cudaError_t launch_encode(const Arena& a, cudaStream_t s);
 // Particles from a.aos (input order) into the state of a single box: positions
 // wrapped into the box, ids the input order; a non-finite coordinate records
-// kFaultNonFinite. And back: positions and canonical velocities (a.vcanon)
-// into a.aos in input order.
+// kFaultNonFinite.
 cudaError_t launch_load_particles(const Arena& a, cudaStream_t s);
-cudaError_t launch_store_particles(const Arena& a, cudaStream_t s);
 cudaError_t launch_decide(const Arena& a, cudaStream_t s, unsigned long long cond_handle);
 cudaError_t launch_rebuild(const Arena& a, cudaStream_t s);
 // The two halves of launch_rebuild: the cell grid (bin, scan, scatter, sort)
@@ -497,7 +495,12 @@ cudaError_t launch_prime(const Arena& a, const CUtensorMap& list_map, bool shift
 cudaError_t launch_step(const Arena& a, const CUtensorMap& list_map, bool shifted_force,
                         cudaStream_t s, unsigned long long next_decision = 0, bool heat = false);
 cudaError_t launch_measure(const Arena& a, const CUtensorMap& list_map, bool shifted_force,
-                           bool canonical, cudaStream_t s);
+                           cudaStream_t s);
+// Positions and canonical velocities of slots first .. first + count - 1 (a
+// whole box) into `out` (count particles on the device, input order), and
+// those slots' vel4.
+cudaError_t launch_read(const Arena& a, const CUtensorMap& list_map, bool shifted_force,
+                        uint32_t first, uint32_t count, double* out, cudaStream_t s);
 // Steps on canonical velocities (one box): begin applies Nose-Hoover's
 // pending scale s2 and this step's s1, kicks and drifts; canon_force computes
 // the forces and then, by `pass`: kPrime records them (and the starting

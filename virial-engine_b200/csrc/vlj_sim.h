@@ -85,6 +85,8 @@ struct vlj_sim {
     cudaGraphNode_t one_decide = nullptr;
     bool one_decide_on = true;
     bool one_ready = false;
+    // the lists were brought up to date and nothing has changed since (lists_now)
+    bool lists_current = false;
     cudaGraphExec_t graph_one_heat = nullptr;  // one step that also takes the pending sample
     cudaGraphExec_t graph_lists = nullptr;  // decide -> IF(rebuild){rebuild chain}
     // per-launch timing of the step kernel (direct launches while on)
