@@ -124,7 +124,8 @@ __global__ void nb_scatter(BinGrid g, const uint32_t* __restrict__ cell_of,
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= g.n) return;
     const uint32_t c = cell_of[i];
-    sorted[cell_start[c] + atomicSub(&counts[c], 1u) - 1u] = i;
+    const uint32_t left = atomicSub(&counts[c], 1u);
+    if (left) sorted[cell_start[c] + left - 1u] = i;  // 0 only where two calls share a scratch
 }
 
 // One warp per cell: each index's rank is the number of smaller indices in
