@@ -1115,12 +1115,14 @@ vlj_status sim_allocate(vlj_sim* s, void* stream) {
     TRY(dalloc(s, &a.cell_start, (size_t)a.ncells + 1));
     TRY(dalloc(s, &a.count, a.ncells));
     {
-        // room for every part of every cell: kMaxParts per cell of a narrow box
+        // room for every part of every cell: kMaxParts per cell of a narrow
+        // box; where few particles rebuild, no more parts than those
         size_t cap = 0;
         for (const Box& b : boxes) {
             const bool narrow = b.cells[0] < 5u || b.cells[1] < 5u || b.cells[2] < 5u;
             cap += (size_t)b.total_cells * (narrow ? kMaxParts : 1u);
         }
+        cap = std::max(cap, (size_t)std::min(n, kSplitSlots));
         if (cap >= (1ull << 32)) return fail(VLJ_INVALID_ARG, "too many cells in all boxes");
         a.work_cap = (uint32_t)cap;
         TRY(dalloc(s, &a.work, cap));

@@ -136,7 +136,7 @@ __global__ void __launch_bounds__(kBuildWarps * 32, kBuildBlocksPerSM) build_lis
         s_q510[t] = __fdiv_rn((float)(t - 256), 510.0f);
     __syncthreads();
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
-    // Warps take home cells (or, in narrow boxes, parts of their home
+    // Warps take home cells (or, where cells split, parts of their home
     // particles) from the step's work list (the non-empty cells of the boxes
     // that rebuild) until it runs out.
     const uint32_t cells = work_total(a), front = a.glob->work_front;
@@ -149,12 +149,11 @@ __global__ void __launch_bounds__(kBuildWarps * 32, kBuildBlocksPerSM) build_lis
         const uint32_t cell = entry >> 3, part = entry & 7u;
         const uint32_t b = box_of_cell(a, cell);
         const Box& bx = a.boxes[b];
-        // this entry's home particles: the whole cell, or part `part` of it
-        // (kPartHomes each, the last part the rest)
+        // this entry's home particles: the whole cell, or its share
         const uint32_t cs0 = a.cell_start[cell], cs1 = a.cell_start[cell + 1];
-        const uint32_t parts = cell_parts(cs1 - cs0, narrow_box(bx));
-        const uint32_t hbeg = parts > 1u ? cs0 + part * kPartHomes : cs0;
-        const uint32_t hend = parts > 1u && part + 1u < parts ? hbeg + kPartHomes : cs1;
+        const uint32_t parts = cell_parts(cs1 - cs0, part_homes(a, narrow_box(bx)));
+        const uint32_t hbeg = cs0 + (cs1 - cs0) * part / parts;
+        const uint32_t hend = cs0 + (cs1 - cs0) * (part + 1u) / parts;
         const uint4* __restrict__ cur = a.cache[a.glob->phase];
         const float dec[3] = {bx.dec[0], bx.dec[1], bx.dec[2]};
         const int32_t n[3] = {(int32_t)bx.cells[0], (int32_t)bx.cells[1], (int32_t)bx.cells[2]};

@@ -51,10 +51,24 @@ __device__ __forceinline__ bool narrow_box(const Box& bx) {
     return bx.cells[0] < 5u || bx.cells[1] < 5u || bx.cells[2] < 5u;
 }
 
-// Work-list entries of a cell of m particles.
-__device__ __forceinline__ uint32_t cell_parts(uint32_t m, bool narrow) {
+// Home particles per work entry where the box's cells split (0: they don't).
+// A warp that builds a whole cell's lists is a chain of some 11,700
+// instructions, 46 us when it runs alone; with few particles to rebuild most
+// of the resident warps would have no cell, so the cells split until the
+// entries are about as many as those warps (some 3,500 on 148 SMs; a second
+// wave costs more than a longer part, and parts round up, hence the 2,400).
+// Every part stages the cell's candidates again, so no further than two
+// homes, and not at all where the cells fill the warps by themselves.
+__device__ __forceinline__ uint32_t part_homes(const Arena& a, bool narrow) {
+    const uint32_t slots = a.glob->rb_slots;
+    if (slots > kSplitSlots) return narrow ? kPartHomes : 0u;
+    return min(kPartHomes, max(2u, (slots + 2399u) / 2400u));
+}
+
+// Work-list entries of a cell of m particles, split by `per` homes.
+__device__ __forceinline__ uint32_t cell_parts(uint32_t m, uint32_t per) {
     if (m == 0u) return 0u;
-    return narrow ? min(kMaxParts, (m + kPartHomes - 1u) / kPartHomes) : 1u;
+    return per ? min(kMaxParts, (m + per - 1u) / per) : 1u;
 }
 
 // ---- cell tiles (tile_step_kernel, and the list build that indexes them) ----

@@ -115,8 +115,8 @@ __global__ void bin_kernel(Arena a) {
 // the counts offset by the box's first slot; counts become zeroed cursors.
 // The box's non-empty cells join the step's work list for the sort and the
 // list build as entries cell * 8 + part: cells of kDenseCell particles or
-// more at its front, the others at its back; in a narrow box every non-empty
-// cell's parts (kPartHomes home particles each) at its front. Each warp takes
+// more at its front, the others at its back; where cells split (part_homes)
+// every non-empty cell's parts at its front. Each warp takes
 // kScanPer runs of 32 consecutive cells, a lane
 // per cell, so every load and store of a run is one coalesced line; shuffles
 // scan within the warp, warp 0 scans the warps' totals, and one atomic per
@@ -137,12 +137,12 @@ __global__ void __launch_bounds__(kScanThreads) scan_kernel(Arena a) {
     if (threadIdx.x == 0) s_carry = bx.first;
     __syncthreads();
     const uint32_t total = bx.total_cells, base = bx.cell_base;
-    const bool narrow = narrow_box(bx);
+    const uint32_t per = part_homes(a, narrow_box(bx));
     for (uint32_t tile = 0; tile < total; tile += (uint32_t)kScanThreads * kScanPer) {
         const uint32_t first = tile + warp * 32u * (uint32_t)kScanPer;
         uint32_t excl[kScanPer];  // within the warp's cells, before this lane's
         // nibble r: front entries of this lane's cell of run r (its parts,
-        // when it holds kDenseCell particles or more or the box is narrow)
+        // when it holds kDenseCell particles or more or cells split)
         unsigned long long front_parts = 0ull;
         uint32_t sparse = 0;      // bit r: one back entry (a cell of fewer, but some)
         uint32_t sum = 0, nd = 0, ns = 0;
@@ -168,9 +168,9 @@ __global__ void __launch_bounds__(kScanThreads) scan_kernel(Arena a) {
             }
             excl[r] = sum + x - v;
             sum += __shfl_sync(0xffffffffu, x, 31);
-            if (narrow) {
+            if (per) {
                 // every non-empty cell's parts go to the front
-                const uint32_t parts = cell_parts(v, true);
+                const uint32_t parts = cell_parts(v, per);
                 front_parts |= (unsigned long long)parts << (4 * r);
                 nd += __reduce_add_sync(0xffffffffu, parts);
             } else {
@@ -227,7 +227,7 @@ __global__ void __launch_bounds__(kScanThreads) scan_kernel(Arena a) {
             // costly cells' parts from the front of the work list, the
             // others from its back
             const uint32_t kd = (uint32_t)(front_parts >> (4 * r)) & 15u;
-            if (narrow) {
+            if (per) {
                 // several parts a cell: an exclusive scan of the counts
                 uint32_t incl = kd;
 #pragma unroll

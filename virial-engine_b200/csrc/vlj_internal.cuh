@@ -84,15 +84,21 @@ constexpr int kSlots = 8;  // measurement accumulators per box
 #endif
 constexpr int kForceThreads = 128;
 constexpr uint32_t kDenseCell = 8;  // particles in a cell the list build takes first
-// In a box under five cells wide on some axis (a batched replica) a cell
-// holds many particles and its candidate stream is most of the box, so its
-// home particles split into parts of kPartHomes (at most kMaxParts, the
-// last taking the rest), each a work-list entry of its own: entry = cell * 8
-// + part.
+// The list build's work entries: a cell's home particles, or a share of them,
+// as entry = cell * 8 + part. In a box under five cells wide on some axis (a
+// batched replica) a cell holds many particles and its candidate stream is
+// most of the box, so its home particles split into parts of about kPartHomes
+// (at most kMaxParts). Where the boxes that rebuild hold no more particles
+// than kSplitSlots, every cell splits, into parts small enough that the
+// entries fill the build's resident warps (part_homes).
 #ifndef VLJ_PART_HOMES
 #define VLJ_PART_HOMES 8
 #endif
 constexpr uint32_t kPartHomes = VLJ_PART_HOMES;
+#ifndef VLJ_SPLIT_SLOTS
+#define VLJ_SPLIT_SLOTS 19200
+#endif
+constexpr uint32_t kSplitSlots = VLJ_SPLIT_SLOTS;
 constexpr uint32_t kMaxParts = 8;
 constexpr int kTileRows = VLJ_TILE_ROWS;
 constexpr int kTileSlots = VLJ_TILE_SLOTS;  // tiles in flight per block
@@ -234,8 +240,8 @@ struct Arena {
     uint32_t* cell_start;  // ncells + 1
     uint32_t* count;
     // the non-empty cells of the boxes that rebuild this step, as entries
-    // cell * 8 + part (one part per cell but in narrow boxes): those of
-    // kDenseCell particles or more and every part of a narrow box's cell
+    // cell * 8 + part (one part per cell unless cells split, part_homes):
+    // those of kDenseCell particles or more and every part of a split cell
     // from the front, the others from the back, so the list build takes the
     // costly work first and ends on cheap work (work_item below)
     uint32_t* work;
