@@ -13,7 +13,8 @@
 namespace vlj {
 
 constexpr int kRing = 3;  // measurement read-back slots (lennard_jones.rs:320)
-constexpr uint32_t kGraphChunk = 16;  // steps per graph launch
+constexpr uint32_t kGraphChunk = 16;  // most steps per graph launch
+constexpr int kChunks = 4;            // graphs of 16, 8, 4 and 2 steps
 
 // One measurement's words as read back into pinned host memory.
 struct Readback {
@@ -72,11 +73,12 @@ struct vlj_sim {
     double* pin_x = nullptr;
     double* pin_v = nullptr;
     uint32_t* pin_id = nullptr;
-    // captured steps: a graph of kGraphChunk steps and one of a single step,
-    // each step's rebuild chain under a conditional node
+    // captured steps: graphs of kGraphChunk >> k steps and one of a single
+    // step, each captured when first needed, each step's rebuild chain under
+    // a conditional node
     bool use_graphs = true;
     cudaStream_t capture_stream = nullptr;
-    cudaGraphExec_t graph_chunk = nullptr;
+    cudaGraphExec_t graph_chunk[vlj::kChunks] = {};
     cudaGraphExec_t graph_one = nullptr;
     // graph_one's template (kept for node updates) and its decide node: while
     // the last step enqueued was graph_one's, whose step kernel took this
