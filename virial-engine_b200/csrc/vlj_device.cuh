@@ -150,6 +150,25 @@ __device__ __forceinline__ bool grid_pass(const Arena& a) {
     return a.glob->any != 0u || a.glob->grid_every_step != 0u;
 }
 
+// One box's rebuild decision in its control words. With `keep` a decision
+// taken at the end of the last step stands, and only a forced rebuild adds
+// to it.
+__device__ __forceinline__ void decide_box(Control& c, float half_skin2, uint32_t reorder_every,
+                                           bool keep) {
+    if (!(keep && c.rebuild)) {
+        const float moved = keep ? 0.0f : __uint_as_float(c.max_disp);
+        const bool rebuild = moved > half_skin2 || c.built == 0u || c.forced != 0u;
+        c.rebuild = rebuild ? 1u : 0u;
+        c.reorder = rebuild && c.rebuilds % reorder_every == 0u ? 1u : 0u;
+        if (rebuild) {
+            c.rebuilds += 1u;
+            c.built = 1u;
+        }
+        if (!keep) c.max_disp = 0u;
+    }
+    c.forced = 0u;
+}
+
 // ---- decide (lennard_jones.wgsl:281-307), by one whole block ----
 // Finishes the previous step's bookkeeping (flip the position copy, advance
 // the step counter), then per box: rebuild when something moved more than
@@ -164,46 +183,44 @@ __device__ __forceinline__ bool grid_pass(const Arena& a) {
 // and only adds the boxes whose rebuild was forced since.
 __device__ __forceinline__ void decide_block(const Arena& a, cudaGraphConditionalHandle handle,
                                              bool set, bool folded = false) {
-    __shared__ int s_any, s_keep;
     Global* g = a.glob;
-    if (folded && a.nboxes == 1u) {
-        // every other block has finished with these words: one thread reads
-        // them all at once and writes the outcome, a single round trip
+    if (a.nboxes == 1u) {
+        // one thread reads all the words at once and writes the outcome: a
+        // single round trip
         if (threadIdx.x != 0) return;
-        Control& c = a.ctrl[0];
+        Control c = a.ctrl[0];
         const Box& bx = a.boxes[0];
-        const uint32_t phase = g->phase, every = g->grid_every_step, built = c.built,
-                       forced = c.forced, rebuilds = c.rebuilds, moved = c.max_disp;
+        const uint32_t phase = g->phase, every = g->grid_every_step, pending = g->pending,
+                       decided = g->decided;
         const unsigned long long step = g->step;
-        const bool rebuild = __uint_as_float(moved) > bx.half_skin2 || built == 0u || forced != 0u;
-        const bool grid = rebuild || every != 0u;
+        const bool keep = !folded && decided != 0u;
+        decide_box(c, bx.half_skin2, bx.reorder_every, keep);
+        a.ctrl[0] = c;
+        const bool grid = c.rebuild != 0u || every != 0u;
         const uint32_t n = grid ? bx.n : 0u;
-        g->phase = phase ^ 1u;
-        g->step = step + 1ull;
-        g->decided = 1u;
+        if (folded || pending) {
+            g->phase = phase ^ 1u;
+            g->step = step + 1ull;
+            g->pending = 0u;
+        }
+        g->decided = folded ? 1u : 0u;
         g->work_front = 0u;
         g->work_back = 0u;
         g->next_build = 0u;
-        c.max_disp = 0u;
-        c.forced = 0u;
-        c.rebuild = rebuild ? 1u : 0u;
-        c.reorder = rebuild && rebuilds % bx.reorder_every == 0u ? 1u : 0u;
-        if (rebuild) {
-            c.rebuilds = rebuilds + 1u;
-            c.built = 1u;
-        }
         a.rb_box[0] = 0u;
         a.rb_first[0] = 0u;
         a.rb_first[grid ? 1 : 0] = n;
         g->rb_boxes = grid ? 1u : 0u;
         g->rb_slots = n;
-        g->any = rebuild ? 1u : 0u;
-        if (set) cudaGraphSetConditional(handle, rebuild ? 1u : 0u);
+        g->any = c.rebuild;
+        if (set) cudaGraphSetConditional(handle, c.rebuild);
         return;
     }
+    __shared__ int s_keep;
+    __shared__ uint32_t s_wbox[32], s_wslot[32], s_cbox, s_cslot;
     if (threadIdx.x == 0) {
-        s_any = 0;
         s_keep = !folded && g->decided != 0u;
+        s_cbox = s_cslot = 0u;
         g->decided = folded ? 1u : 0u;
         g->work_front = 0u;
         g->work_back = 0u;
@@ -214,57 +231,38 @@ __device__ __forceinline__ void decide_block(const Arena& a, cudaGraphConditiona
             g->pending = 0u;
         }
     }
+    // Each pass decides blockDim.x boxes, a thread each, and compacts those
+    // that rebuild in box order, with their particle counts summed before
+    // each (two block-wide exclusive scans); the next pass's words load
+    // behind it. A pass that read the decisions back in a second loop took
+    // 8.7 us for 512 boxes.
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+    Control next_c = {};
+    float next_skin = 0.0f;
+    uint32_t next_every = 1u, next_n = 0u;
+    auto fetch = [&](uint32_t b) {
+        if (b >= a.nboxes) return;
+        next_c = a.ctrl[b];
+        next_skin = a.boxes[b].half_skin2;
+        next_every = a.boxes[b].reorder_every;
+        next_n = a.boxes[b].n;
+    };
+    fetch(threadIdx.x);
     __syncthreads();
     const bool keep = s_keep != 0;
-    for (uint32_t b = threadIdx.x; b < a.nboxes; b += blockDim.x) {
-        Control& c = a.ctrl[b];
-        const Box& bx = a.boxes[b];
-        if (keep && c.rebuild) {
-            // decided at the end of the last step
-            c.forced = 0u;
-            s_any = 1;
-            continue;
-        }
-        const float moved = keep ? 0.0f : __uint_as_float(c.max_disp);
-        if (!keep) c.max_disp = 0u;
-        const bool rebuild = moved > bx.half_skin2 || c.built == 0u || c.forced != 0u;
-        c.forced = 0u;
-        c.rebuild = rebuild ? 1u : 0u;
-        if (rebuild) {
-            c.reorder = (c.rebuilds % bx.reorder_every == 0u) ? 1u : 0u;
-            c.rebuilds += 1u;
-            c.built = 1u;
-            s_any = 1;
-        } else {
-            c.reorder = 0u;
-        }
-    }
-    __syncthreads();
-    if (a.nboxes == 1u) {
-        if (threadIdx.x == 0) {
-            // the particles the grid kernels cover: the box's, when its lists
-            // rebuild or its grid is rebuilt every step
-            const bool r = a.ctrl[0].rebuild != 0u || g->grid_every_step != 0u;
-            a.rb_box[0] = 0u;
-            a.rb_first[0] = 0u;
-            a.rb_first[r ? 1 : 0] = r ? a.boxes[0].n : 0u;
-            g->rb_boxes = r ? 1u : 0u;
-            g->rb_slots = r ? a.boxes[0].n : 0u;
-            g->any = (uint32_t)s_any;
-            if (set) cudaGraphSetConditional(handle, (unsigned)s_any);
-        }
-        return;
-    }
-    // the rebuilding boxes, compacted in box order, with their particle counts
-    // summed before each: two block-wide exclusive scans per pass
-    __shared__ uint32_t s_wbox[32], s_wslot[32], s_cbox, s_cslot;
-    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
-    if (threadIdx.x == 0) s_cbox = s_cslot = 0u;
-    __syncthreads();
     for (uint32_t base = 0; base < a.nboxes; base += blockDim.x) {
         const uint32_t b = base + threadIdx.x;
-        const bool flag = b < a.nboxes && a.ctrl[b].rebuild != 0u;
-        const uint32_t nb = flag ? a.boxes[b].n : 0u;
+        Control c = next_c;
+        const float skin2 = next_skin;
+        const uint32_t every = next_every, n = next_n;
+        fetch(b + blockDim.x);
+        bool flag = false;
+        if (b < a.nboxes) {
+            decide_box(c, skin2, every, keep);
+            a.ctrl[b] = c;
+            flag = c.rebuild != 0u;
+        }
+        const uint32_t nb = flag ? n : 0u;
         uint32_t ib = flag ? 1u : 0u, is = nb;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
@@ -303,8 +301,8 @@ __device__ __forceinline__ void decide_block(const Arena& a, cudaGraphConditiona
         a.rb_first[s_cbox] = s_cslot;
         g->rb_boxes = s_cbox;
         g->rb_slots = s_cslot;
-        g->any = (uint32_t)s_any;
-        if (set) cudaGraphSetConditional(handle, (unsigned)s_any);
+        g->any = s_cbox ? 1u : 0u;
+        if (set) cudaGraphSetConditional(handle, s_cbox ? 1u : 0u);
     }
 }
 

@@ -444,10 +444,11 @@ cudaError_t launch_load_particles(const Arena& a, cudaStream_t s) {
 }
 
 cudaError_t launch_decide(const Arena& a, cudaStream_t s, unsigned long long cond_handle) {
+    const unsigned threads = a.nboxes == 1u ? 32u : 512u;  // a single box takes one thread
     if (cond_handle)
-        decide_kernel<true><<<1, kBlock, 0, s>>>(a, (cudaGraphConditionalHandle)cond_handle);
+        decide_kernel<true><<<1, threads, 0, s>>>(a, (cudaGraphConditionalHandle)cond_handle);
     else
-        decide_kernel<false><<<1, kBlock, 0, s>>>(a, (cudaGraphConditionalHandle)0);
+        decide_kernel<false><<<1, threads, 0, s>>>(a, (cudaGraphConditionalHandle)0);
     return after_launch();
 }
 
