@@ -1067,6 +1067,7 @@ vlj_status sim_allocate(vlj_sim* s, void* stream) {
         b.cell_base = (uint32_t)cells;
         slots += b.n;
         cells += b.total_cells;
+        a.max_cells = std::max(a.max_cells, b.total_cells);
         cap = std::max(cap, b.capacity);
     }
     if (slots >= (1ull << 30)) return fail(VLJ_INVALID_ARG, "at most 2^30 - 1 particles in all");

@@ -29,7 +29,7 @@ __device__ __forceinline__ uint32_t box_of_cell(const Arena& a, uint32_t cell) {
 // Every kernel counts its own launch once, so the number of this library's
 // kernels that ran (graph nodes skipped by a condition do not) is exact.
 __device__ __forceinline__ void count_kernel(const Arena& a) {
-    if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&a.glob->kernels, 1ull);
+    if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) atomicAdd(&a.glob->kernels, 1ull);
 }
 
 __device__ __forceinline__ bool rebuilding(const Arena& a, uint32_t b) {

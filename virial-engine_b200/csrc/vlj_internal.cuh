@@ -25,7 +25,7 @@
 //             one load and a warp reads 512 contiguous bytes; the force
 //             kernels stream rows per thread past L1 (or, as a tuning option,
 //             stage row tiles into shared memory with TMA).
-//   cells     per cell: count (atomic cursor) and start. Boxes own contiguous
+//   cells     per cell: count (zero between rebuilds) and start. Boxes own contiguous
 //             runs of slots and cells, so one start array of ncells + 1 entries
 //             serves every box: box b's last cell ends where box b + 1 begins.
 //   work      per step, the non-empty cells of the rebuilding boxes; rb_box /
@@ -228,6 +228,7 @@ struct Arena {
     uint32_t nslots;     // particles in all boxes
     uint32_t seg;        // padded slot count (list row length)
     uint32_t ncells;     // cells in all boxes
+    uint32_t max_cells;  // cells of the box with the most
     const uint32_t* box_of_slot;  // null for a single box
     const uint32_t* box_of_cell;  // null for a single box
     double* x;
