@@ -187,14 +187,12 @@ vlj_status upload_particles(vlj_sim* s, const vlj_particle* p, size_t count) {
     CUDA_TRY(cudaMemcpyAsync(s->arena.aos, p, sizeof(vlj_particle) * count, cudaMemcpyHostToDevice,
                              s->stream));
     CUDA_TRY(launch_load_particles(s->arena, s->stream));
-    Global g;
-    CUDA_TRY(cudaMemcpyAsync(&g, s->arena.glob, sizeof g, cudaMemcpyDeviceToHost, s->stream));
-    CUDA_TRY(cudaStreamSynchronize(s->stream));
-    if (g.fault == kFaultNonFinite) {
+    const vlj_status st = sim_read_status(s);
+    if (s->status_glob()->fault == kFaultNonFinite) {
         cudaMemsetAsync(&s->arena.glob->fault, 0, sizeof(uint32_t), s->stream);
         return fail(VLJ_INVALID_ARG, "a particle has a non-finite coordinate");
     }
-    return VLJ_OK;
+    return st;
 }
 
 // The rebuild decision, and the rebuild where it is due, ahead of a pass over
@@ -220,15 +218,12 @@ vlj_status restart(vlj_sim* s, const vlj_particle* p, size_t count) {
     s->one_ready = false;
     s->lists_current = false;
     TRY(upload_particles(s, p, count));
-    uint32_t one = 1u;
-    CUDA_TRY(cudaMemcpyAsync(&s->arena.ctrl[0].forced, &one, sizeof one, cudaMemcpyHostToDevice,
-                             s->stream));
+    CUDA_TRY(cudaMemsetAsync(&s->arena.ctrl[0].forced, 1, sizeof(uint32_t), s->stream));
     CUDA_TRY(launch_decide(s->arena, s->stream, 0));
     CUDA_TRY(launch_encode(s->arena, s->stream));
     CUDA_TRY(launch_rebuild(s->arena, s->stream));
     // lists that overflowed on the first build grow before the first forces
-    bool grew = false;
-    TRY(sim_grow_lists(s, &grew));
+    TRY(sim_settle(s));
     if (s->canonical()) {
         // the thermostat starts at rest (xi = eta = 0) from the given
         // velocities; the first forces are recorded for the first half kick
@@ -279,13 +274,7 @@ vlj_status enqueue_measure(vlj_sim* s, int slot) {
     CUDA_TRY(launch_measure(s->arena, s->list_map, s->shifted_force, s->stream));
     if (s->box.drawn == VLJ_DRAWN_TEMPERATURE) CUDA_TRY(launch_drawn_temperature(s->arena, s->stream));
     Readback* r = &s->ring[slot];
-    CUDA_TRY(cudaMemcpyAsync(r->slots, s->arena.accum, sizeof(r->slots), cudaMemcpyDeviceToHost,
-                             s->stream));
-    CUDA_TRY(cudaMemcpyAsync(&r->ctrl, s->arena.ctrl, sizeof(Control), cudaMemcpyDeviceToHost,
-                             s->stream));
-    if (s->nose_hoover)
-        CUDA_TRY(cudaMemcpyAsync(&r->nh, s->arena.nh, sizeof(Thermo), cudaMemcpyDeviceToHost,
-                                 s->stream));
+    CUDA_TRY(cudaMemcpyAsync(r, s->arena.accum, sizeof(Readback), cudaMemcpyDeviceToHost, s->stream));
     CUDA_TRY(cudaEventRecord(s->ring_event[slot], s->stream));
     s->ring_busy[slot] = true;
     s->ring_step[slot] = s->steps;
@@ -311,6 +300,7 @@ vlj_sim::~vlj_sim() {
     for (int k = 0; k < kRing; k++)
         if (ring_event[k]) cudaEventDestroy(ring_event[k]);
     if (ring) cudaFreeHost(ring);
+    if (status) cudaFreeHost(status);
     for (void* p : allocations) cudaFree(p);
     if (own_stream && stream) cudaStreamDestroy(stream);
 }
@@ -398,10 +388,7 @@ vlj_status vlj_run(vlj_sim* s, uint64_t steps) {
         TRY(vlj_step(s, batch));
         steps -= batch;
     }
-    CUDA_TRY(cudaStreamSynchronize(s->stream));
-    TRY(check_fault(s));
-    bool grew = false;
-    return sim_grow_lists(s, &grew);
+    return sim_settle(s);
 }
 
 vlj_status vlj_measure(vlj_sim* s, int* accepted) {
@@ -437,6 +424,7 @@ vlj_status vlj_poll(vlj_sim* s, vlj_measurement* out, size_t capacity, size_t* w
         if (n >= capacity || !out) break;
         out[n] = decode(s, s->ring[r.second], r.first);
         if (out[n].list_overflow && s->list_growth) s->grow_pending = true;
+        if (s->ring[r.second].glob.fault) s->polled_fault = s->ring[r.second].glob.fault;
         n++;
         s->ring_busy[r.second] = false;
     }
@@ -455,7 +443,9 @@ vlj_status vlj_measure_now(vlj_sim* s, vlj_measurement* out) {
     TRY(vlj_poll(s, buf, kRing, &n));
     if (n == 0) return fail(VLJ_CUDA_ERROR, "the measurement did not finish");
     *out = buf[n - 1];
-    TRY(check_fault(s));
+    const uint32_t fault = s->polled_fault;
+    s->polled_fault = 0;
+    TRY(fault_status(fault));
     if (out->list_overflow && s->list_growth) {
         // lists that dropped pairs: grow them, rebuild, measure again
         bool grew = false;
@@ -472,8 +462,7 @@ vlj_status vlj_read_particles(vlj_sim* s, vlj_particle* out) {
     if (s->box.drawn == VLJ_DRAWN_TEMPERATURE) CUDA_TRY(launch_drawn_temperature(s->arena, s->stream));
     CUDA_TRY(cudaMemcpyAsync(out, s->arena.aos, sizeof(vlj_particle) * s->n, cudaMemcpyDeviceToHost,
                              s->stream));
-    CUDA_TRY(cudaStreamSynchronize(s->stream));
-    return check_fault(s);
+    return sim_read_status(s);
 }
 
 vlj_status vlj_write_particles(vlj_sim* s, const vlj_particle* p, size_t count) {
@@ -984,13 +973,28 @@ vlj_status make_list_map(const Arena& a, uint32_t rows, CUtensorMap* out) {
 }
 
 // VLJ_TIMEOUT when a kernel recorded a fault (a TMA tile that never arrived).
-vlj_status check_fault(vlj_sim* s) {
-    Global g;
-    CUDA_TRY(cudaMemcpyAsync(&g, s->arena.glob, sizeof g, cudaMemcpyDeviceToHost, s->stream));
-    CUDA_TRY(cudaStreamSynchronize(s->stream));
-    if (g.fault == kFaultTmaTimeout)
+vlj_status fault_status(uint32_t fault) {
+    if (fault == kFaultTmaTimeout)
         return fail(VLJ_TIMEOUT, "a list tile did not arrive within the wait limit");
-    if (g.fault) return fail(VLJ_CUDA_ERROR, "kernel fault code %u", g.fault);
+    if (fault) return fail(VLJ_CUDA_ERROR, "kernel fault code %u", fault);
+    return VLJ_OK;
+}
+
+vlj_status sim_read_status(vlj_sim* s) {
+    CUDA_TRY(cudaMemcpyAsync(s->status, s->arena.accum, s->status_bytes, cudaMemcpyDeviceToHost, s->stream));
+    CUDA_TRY(cudaStreamSynchronize(s->stream));
+    return fault_status(s->status_glob()->fault);
+}
+
+vlj_status sim_settle(vlj_sim* s) {
+    TRY(sim_read_status(s));
+    s->grow_pending = false;
+    const Control* c = s->status_ctrl();
+    for (uint32_t b = 0; b < s->arena.nboxes; b++)
+        if (c[b].overflow > (s->replicas.empty() ? s->box : s->replicas[b]).capacity) {
+            bool grew = false;
+            return sim_grow_lists(s, &grew);
+        }
     return VLJ_OK;
 }
 
@@ -1088,8 +1092,19 @@ vlj_status sim_allocate(vlj_sim* s, void* stream) {
     Box* d_box = nullptr;
     TRY(dalloc(s, &d_box, boxes.size()));
     a.boxes = d_box;
-    TRY(dalloc(s, &a.ctrl, boxes.size()));
-    TRY(dalloc(s, &a.glob, 1));
+    // the words the host reads back lie side by side (Readback)
+    {
+        const size_t nb = boxes.size();
+        s->status_bytes = nb * (sizeof(long long) * kSlots + sizeof(Control) + sizeof(Thermo)) + sizeof(Global);
+        unsigned char* words = nullptr;
+        TRY(dalloc(s, &words, s->status_bytes));
+        a.accum = reinterpret_cast<unsigned long long*>(words);
+        a.ctrl = reinterpret_cast<Control*>(a.accum + nb * kSlots);
+        a.nh = reinterpret_cast<Thermo*>(a.ctrl + nb);
+        a.glob = reinterpret_cast<Global*>(a.nh + nb);
+        CUDA_TRY(cudaMallocHost(&s->status, s->status_bytes));
+        std::memset(s->status, 0, s->status_bytes);
+    }
     if (batched) {
         std::vector<uint32_t> of_slot(seg, 0u), of_cell(a.ncells);
         for (uint32_t b = 0; b < a.nboxes; b++) {
@@ -1151,8 +1166,6 @@ vlj_status sim_allocate(vlj_sim* s, void* stream) {
     TRY(dalloc(s, &a.sv, 3 * (size_t)seg));
     TRY(dalloc(s, &a.sid, seg));
     TRY(dalloc(s, &a.scell, seg));
-    TRY(dalloc(s, &a.accum, (size_t)kSlots * boxes.size()));
-    TRY(dalloc(s, &a.nh, boxes.size()));
     TRY(dalloc(s, &a.hex, 1));
     TRY(dalloc(s, &a.acc, seg));
     TRY(dalloc(s, &a.pe_half, 2 * (size_t)seg));
@@ -1164,12 +1177,14 @@ vlj_status sim_allocate(vlj_sim* s, void* stream) {
     CUDA_TRY(cudaMemcpy(a.cell_start + a.ncells, &n, sizeof n, cudaMemcpyHostToDevice));
     CUDA_TRY(cudaMemcpy(d_box, boxes.data(), sizeof(Box) * boxes.size(), cudaMemcpyHostToDevice));
     CUDA_TRY(cudaMallocHost(&s->ring, sizeof(Readback) * kRing));
-    CUDA_TRY(cudaMallocHost(&s->pin_x, sizeof(double) * 3 * (size_t)seg));
-    CUDA_TRY(cudaMallocHost(&s->pin_v, sizeof(double) * 3 * (size_t)seg));
-    CUDA_TRY(cudaMallocHost(&s->pin_id, sizeof(uint32_t) * (size_t)seg));
-    std::memset(s->pin_x, 0, sizeof(double) * 3 * (size_t)seg);
-    std::memset(s->pin_v, 0, sizeof(double) * 3 * (size_t)seg);
-    std::memset(s->pin_id, 0, sizeof(uint32_t) * (size_t)seg);
+    if (batched) {
+        CUDA_TRY(cudaMallocHost(&s->pin_x, sizeof(double) * 3 * (size_t)seg));
+        CUDA_TRY(cudaMallocHost(&s->pin_v, sizeof(double) * 3 * (size_t)seg));
+        CUDA_TRY(cudaMallocHost(&s->pin_id, sizeof(uint32_t) * (size_t)seg));
+        std::memset(s->pin_x, 0, sizeof(double) * 3 * (size_t)seg);
+        std::memset(s->pin_v, 0, sizeof(double) * 3 * (size_t)seg);
+        std::memset(s->pin_id, 0, sizeof(uint32_t) * (size_t)seg);
+    }
     CUDA_TRY(cudaStreamCreateWithFlags(&s->capture_stream, cudaStreamNonBlocking));
     for (int k = 0; k < kRing; k++) {
         CUDA_TRY(cudaEventCreateWithFlags(&s->ring_event[k], cudaEventDisableTiming));

@@ -67,8 +67,7 @@ vlj_status vlj_read_profile(vlj_sim* s, vlj_slab* slabs, double virial[3], uint6
     std::vector<long long> raw((size_t)bins * 8 + 3);
     CUDA_TRY(cudaMemcpyAsync(raw.data(), s->arena.profile, raw.size() * sizeof(long long),
                              cudaMemcpyDeviceToHost, s->stream));
-    CUDA_TRY(cudaStreamSynchronize(s->stream));
-    TRY(check_fault(s));
+    TRY(sim_read_status(s));
     const double n = (double)s->profile_samples;
     const double width = s->box.box[2] / (double)bins;
     auto q = [&](size_t w) { return n > 0.0 ? (double)raw[w] / kOne / n : 0.0; };
@@ -138,8 +137,7 @@ vlj_status vlj_read_heat_current(vlj_sim* s, double* out, size_t capacity, size_
     std::vector<long long> raw(1 + 3 * n);
     CUDA_TRY(cudaMemcpyAsync(raw.data(), s->series, raw.size() * sizeof(long long),
                              cudaMemcpyDeviceToHost, s->stream));
-    CUDA_TRY(cudaStreamSynchronize(s->stream));
-    TRY(check_fault(s));
+    TRY(sim_read_status(s));
     const size_t m = std::min(n, capacity);
     for (size_t k = 0; k < m && out; k++)
         for (int c = 0; c < 3; c++) out[3 * k + c] = (double)raw[1 + 3 * k + c] / kOne;

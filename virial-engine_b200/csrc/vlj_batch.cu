@@ -42,15 +42,11 @@ using namespace vlj;
 
 struct vlj_batch {
     vlj_sim* sim = nullptr;
-    long long* accum = nullptr;  // pinned: kSlots per replica
-    Control* ctrl = nullptr;     // pinned: one per replica
     ~vlj_batch() {
         if (sim) {
             if (sim->stream) cudaStreamSynchronize(sim->stream);
             delete sim;
         }
-        if (accum) cudaFreeHost(accum);
-        if (ctrl) cudaFreeHost(ctrl);
     }
 };
 
@@ -180,9 +176,6 @@ vlj_status vlj_batch_create(const vlj_replica_desc* replicas, size_t count, doub
         }
     }
     if (st == VLJ_OK) st = sim_allocate(s, stream);
-    if (st == VLJ_OK && (cudaMallocHost(&bt->accum, sizeof(long long) * kSlots * count) != cudaSuccess ||
-                         cudaMallocHost(&bt->ctrl, sizeof(Control) * count) != cudaSuccess))
-        st = fail(VLJ_CUDA_ERROR, "pinned read-back buffers");
     if (st == VLJ_OK) st = upload(s, replicas);
     if (st == VLJ_OK) {
         // never built: every box rebuilds at the first decision
@@ -190,15 +183,14 @@ vlj_status vlj_batch_create(const vlj_replica_desc* replicas, size_t count, doub
         if (e == cudaSuccess) e = launch_encode(s->arena, s->stream);
         if (e == cudaSuccess) e = launch_rebuild(s->arena, s->stream);
         // lists that overflowed on the first build grow before the first forces
-        bool grew = false;
-        if (e == cudaSuccess) st = sim_grow_lists(s, &grew);
+        if (e == cudaSuccess) st = sim_settle(s);
         if (st != VLJ_OK) e = cudaErrorUnknown;
         if (e == cudaSuccess) e = launch_prime(s->arena, s->list_map, s->shifted_force, s->stream);
         if (e == cudaSuccess) e = cudaStreamSynchronize(s->stream);
         if (e != cudaSuccess && st == VLJ_OK)
             st = fail(VLJ_CUDA_ERROR, "first lists: %s", cudaGetErrorString(e));
     }
-    if (st == VLJ_OK) st = check_fault(s);
+    if (st == VLJ_OK) st = sim_read_status(s);
     if (st != VLJ_OK) {
         delete bt;
         return st;
@@ -230,10 +222,7 @@ vlj_status vlj_batch_run(vlj_batch* bt, uint64_t steps) {
         TRY(vlj_batch_step(bt, chunk));
         steps -= chunk;
     }
-    CUDA_TRY(cudaStreamSynchronize(bt->sim->stream));
-    TRY(check_fault(bt->sim));
-    bool grew = false;
-    return sim_grow_lists(bt->sim, &grew);
+    return sim_settle(bt->sim);
 }
 
 vlj_status vlj_batch_measure(vlj_batch* bt, vlj_measurement* out) {
@@ -241,14 +230,10 @@ vlj_status vlj_batch_measure(vlj_batch* bt, vlj_measurement* out) {
     vlj_sim* s = bt->sim;
     const size_t boxes = s->replicas.size();
     TRY(measure_all(bt));
-    CUDA_TRY(cudaMemcpyAsync(bt->accum, s->arena.accum, sizeof(long long) * kSlots * boxes,
-                             cudaMemcpyDeviceToHost, s->stream));
-    CUDA_TRY(cudaMemcpyAsync(bt->ctrl, s->arena.ctrl, sizeof(Control) * boxes,
-                             cudaMemcpyDeviceToHost, s->stream));
-    CUDA_TRY(cudaStreamSynchronize(s->stream));
-    TRY(check_fault(s));
+    TRY(sim_read_status(s));
+    const Control* ctrl = s->status_ctrl();
     bool overflow = false;
-    for (size_t r = 0; r < boxes; r++) overflow = overflow || bt->ctrl[r].overflow != 0u;
+    for (size_t r = 0; r < boxes; r++) overflow = overflow || ctrl[r].overflow != 0u;
     if (overflow && s->list_growth) {
         // lists that dropped pairs: grow them, rebuild, measure again
         bool grew = false;
@@ -256,7 +241,7 @@ vlj_status vlj_batch_measure(vlj_batch* bt, vlj_measurement* out) {
         if (grew) return vlj_batch_measure(bt, out);
     }
     for (size_t r = 0; r < boxes; r++)
-        out[r] = decode(s, s->replicas[r], bt->accum + kSlots * r, bt->ctrl[r]);
+        out[r] = decode(s, s->replicas[r], s->status_slots() + kSlots * r, ctrl[r]);
     return VLJ_OK;
 }
 
@@ -271,7 +256,7 @@ vlj_status vlj_batch_read_particles(vlj_batch* bt, size_t replica, vlj_particle*
     CUDA_TRY(launch_read(s->arena, s->list_map, s->shifted_force, bx.first, bx.n, s->arena.aos, s->stream));
     CUDA_TRY(cudaMemcpyAsync(out, s->arena.aos, sizeof(vlj_particle) * bx.n, cudaMemcpyDeviceToHost,
                              s->stream));
-    TRY(check_fault(s));
+    TRY(sim_read_status(s));
     return VLJ_OK;
 }
 

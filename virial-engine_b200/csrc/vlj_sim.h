@@ -16,12 +16,17 @@ constexpr int kRing = 3;  // measurement read-back slots (lennard_jones.rs:320)
 constexpr uint32_t kGraphChunk = 16;  // most steps per graph launch
 constexpr int kChunks = 4;            // graphs of 16, 8, 4 and 2 steps
 
-// One measurement's words as read back into pinned host memory.
+// The words the host reads back, one after the other on the device (the
+// measurement sums, control words and thermostats of every box, then the
+// arena's global words), so that one copy brings them all. For a single box:
 struct Readback {
     long long slots[kSlots];
     Control ctrl;
     Thermo nh;
+    Global glob;
 };
+static_assert(sizeof(Readback) == sizeof(long long) * kSlots + sizeof(Control) + sizeof(Thermo) + sizeof(Global),
+              "the words lie side by side");
 
 double scale_for(double magnitude);
 vlj_status check_settings(const vlj_settings* st);
@@ -59,6 +64,18 @@ struct vlj_sim {
     cudaEvent_t ring_event[vlj::kRing] = {};
     bool ring_busy[vlj::kRing] = {};
     uint64_t ring_step[vlj::kRing] = {};
+    // those words of every box, pinned (sim_read_status), and a fault that a
+    // polled measurement came with
+    unsigned char* status = nullptr;
+    size_t status_bytes = 0;
+    uint32_t polled_fault = 0;
+    const long long* status_slots() const { return reinterpret_cast<const long long*>(status); }
+    const vlj::Control* status_ctrl() const {
+        return reinterpret_cast<const vlj::Control*>(status + sizeof(long long) * vlj::kSlots * arena.nboxes);
+    }
+    const vlj::Global* status_glob() const {
+        return reinterpret_cast<const vlj::Global*>(status + status_bytes - sizeof(vlj::Global));
+    }
     // profiles
     uint64_t profile_samples = 0;
     // heat current series
@@ -69,7 +86,7 @@ struct vlj_sim {
     bool heat_pending = false;
     uint32_t series_capacity = 0;
     unsigned long long* series = nullptr;  // owned here (reallocated by record)
-    // pinned staging for particle uploads and read-backs (x, v: 3 * seg; id: seg)
+    // pinned staging for a batch's particle uploads (x, v: 3 * seg; id: seg)
     double* pin_x = nullptr;
     double* pin_v = nullptr;
     uint32_t* pin_id = nullptr;
@@ -104,7 +121,12 @@ vlj_status sim_allocate(vlj_sim* s, void* stream);
 vlj_status make_list_map(const Arena& a, uint32_t rows, CUtensorMap* out);
 // Decide and, when due, rebuild the lists now (positions are about to be read).
 vlj_status sim_lists_now(vlj_sim* s);
-vlj_status check_fault(vlj_sim* s);
+// Everything enqueued so far, then the status words, waited for; an error
+// where a kernel recorded a fault.
+vlj_status sim_read_status(vlj_sim* s);
+vlj_status fault_status(uint32_t fault);
+// The same, and lists that overflowed grow: what ends a run.
+vlj_status sim_settle(vlj_sim* s);
 vlj_status sim_enqueue_steps(vlj_sim* s, uint32_t steps);
 // Takes a pending heat-current sample now, with the sampling kernel.
 vlj_status sim_flush_heat(vlj_sim* s);
