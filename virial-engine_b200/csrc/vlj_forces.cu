@@ -79,13 +79,6 @@ __device__ __forceinline__ void finish_part(PairSums& s) {
     }
 }
 
-// A 32-bit integer as f64, exactly, by its bits in the fraction of 2^52 +
-// 2^31: an f64 subtraction in place of the conversion, whose unit takes a
-// quarter of the FP64 pipe's rate.
-__device__ __forceinline__ double int_to_double(uint32_t x) {
-    return __dsub_rn(__hiloint2double(0x43300000, (int)(x ^ 0x80000000u)), 4503601774854144.0);
-}
-
 __device__ __forceinline__ void add_force(PairSums& s, float dx, float dy, float dz, float f) {
     s.px = __fmaf_rn(-dx, f, s.px);
     s.py = __fmaf_rn(-dy, f, s.py);
@@ -202,9 +195,9 @@ __device__ __forceinline__ void pair_terms(PairSums& s, const uint4 own, const u
         // integer differences times the box step are exact in f64): on a
         // lattice, where every pair at one distance rounds alike, the f32
         // components' three roundings would bias the virial coherently.
-        const double ex = int_to_double(pj.x - own.x) * (double)dec0;
-        const double ey = int_to_double(pj.y - own.y) * (double)dec1;
-        const double ez = int_to_double(pj.z - own.z) * (double)dec2;
+        const double ex = (double)(int32_t)(pj.x - own.x) * (double)dec0;
+        const double ey = (double)(int32_t)(pj.y - own.y) * (double)dec1;
+        const double ez = (double)(int32_t)(pj.z - own.z) * (double)dec2;
         float rf, u, t, e;
         lj_pair<SHIFTED_FORCE>((float)__fma_rn(ez, ez, __fma_rn(ey, ey, __dmul_rn(ex, ex))), bx, rf, u);
         two_sum(s.ppe, 0.5f * u, t, e);
