@@ -121,6 +121,7 @@ __device__ __forceinline__ bool repeats(int32_t d, int32_t n) {
 template <bool TILES>
 __global__ void __launch_bounds__(kBuildWarps * 32, kBuildBlocksPerSM) build_list_kernel(Arena a) {
     constexpr int kStage = TILES ? kStageTiles : vlj::kStage;
+    chain_wait();
     count_kernel(a);
     if (!a.glob->any) return;
     // the tile step kernel reads the 16-bit lists from the next step on
@@ -465,10 +466,8 @@ __global__ void __launch_bounds__(kBuildWarps * 32, kBuildBlocksPerSM) build_lis
 cudaError_t launch_build_list(const Arena& a, cudaStream_t s) {
     const unsigned blocks = (unsigned)sm_count() * kBuildBlocksPerSM;
     if (a.list16)
-        build_list_kernel<true><<<blocks, kBuildWarps * 32, 0, s>>>(a);
-    else
-        build_list_kernel<false><<<blocks, kBuildWarps * 32, 0, s>>>(a);
-    return cudaGetLastError();
+        return launch_chained(build_list_kernel<true>, dim3(blocks), kBuildWarps * 32, s, a);
+    return launch_chained(build_list_kernel<false>, dim3(blocks), kBuildWarps * 32, s, a);
 }
 
 }  // namespace vlj

@@ -18,6 +18,33 @@ cudaError_t after_launch(unsigned n = 1);
 int sm_count();
 cudaError_t launch_build_list(const Arena& a, cudaStream_t s);  // vlj_build.cu
 
+// Chained launches: a kernel launched with launch_chained may start while the
+// kernel before it on the stream still runs (its blocks are placed, its first
+// instructions fetched) and waits in chain_wait, before it touches memory,
+// until that one has finished and its writes are seen; chain_next in the one
+// before says from when. Every kernel of a chain waits, so each also follows
+// all before it. In the others chain_wait and chain_next do nothing.
+// The kernels of a rebuild and of a canonical step are a few microseconds each
+// and the launch gap between two of them about one: 40 Nose-Hoover steps at
+// 15,600 atoms take 1,263 us with plain launches and 1,207 so, 50 exchange steps
+// 1,501 and 1,465, 100 steps of 32 replicas 16.55 and 16.37 ms.
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void chain_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+template <class... P, class... A>
+cudaError_t launch_chained(void (*kernel)(P...), dim3 grid, unsigned threads, cudaStream_t s, A... args) {
+    cudaLaunchConfig_t c = {};
+    c.gridDim = grid;
+    c.blockDim = dim3(threads);
+    c.stream = s;
+    cudaLaunchAttribute at = {};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    c.attrs = &at;
+    c.numAttrs = 1;
+    return cudaLaunchKernelEx(&c, kernel, args...);
+}
+
 __device__ __forceinline__ uint32_t box_of_slot(const Arena& a, uint32_t slot) {
     return a.box_of_slot ? a.box_of_slot[slot] : 0u;
 }

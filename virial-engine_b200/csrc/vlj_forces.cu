@@ -1,7 +1,8 @@
 // CUDA kernels of the pair forces, the integrator and the measurements,
 // sm_100a.
 //
-// One thread per particle, 128 per block. Each thread reads its Verlet-list
+// One thread per particle, 128 per block (small grids: several lanes per
+// particle, lanes_for). Each thread reads its Verlet-list
 // rows (a row is four entries of a particle, 16 B; a warp's rows are 512
 // contiguous bytes) one ahead with loads that do not allocate in L1, issues
 // the four neighbour gathers of a row through L1 together, then does the four
@@ -1000,6 +1001,8 @@ __global__ void __launch_bounds__(kForceThreads) read_kernel(Arena a, const __gr
 // begin: every thread takes the start half step from the same state, so all
 // of them compute the same s1; the box's first thread stores the result.
 __global__ void __launch_bounds__(kBlock) begin_kernel(Arena a) {
+    chain_next();
+    chain_wait();
     count_kernel(a);
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     const bool valid = i < a.nslots;
@@ -1115,6 +1118,7 @@ __device__ __forceinline__ long long warp_sum(long long x) {
 template <bool SHIFTED_FORCE, int PASS, int LANES>
 __global__ void __launch_bounds__(kForceThreads) canon_force_kernel(Arena a,
                                                                     const __grid_constant__ CUtensorMap map) {
+    chain_next();
     count_kernel(a);
     constexpr int kWarps = kForceThreads / 32;
     __shared__ __align__(128) Stage st;
@@ -1225,6 +1229,8 @@ __global__ void __launch_bounds__(kForceThreads) canon_force_kernel(Arena a,
 // v <- v + (s - 1)(v - v_com); the moved positions go back into the current
 // position copy.
 __global__ void __launch_bounds__(kBlock) hex_apply_kernel(Arena a) {
+    chain_next();
+    chain_wait();
     count_kernel(a);
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= a.nslots) return;
@@ -1517,8 +1523,8 @@ cudaError_t launch_read(const Arena& a, const CUtensorMap& map, bool shifted_for
 }
 
 cudaError_t launch_begin(const Arena& a, cudaStream_t s) {
-    begin_kernel<<<blocks_for(a.nslots), kBlock, 0, s>>>(a);
-    return after_launch();
+    const cudaError_t e = launch_chained(begin_kernel, dim3(blocks_for(a.nslots)), kBlock, s, a);
+    return e != cudaSuccess ? e : after_launch();
 }
 
 template <bool SF, int PASS, int LANES>
@@ -1566,8 +1572,8 @@ cudaError_t launch_canon_force(const Arena& a, const CUtensorMap& map, bool shif
 }
 
 cudaError_t launch_hex_apply(const Arena& a, cudaStream_t s) {
-    hex_apply_kernel<<<blocks_for(a.nslots), kBlock, 0, s>>>(a);
-    return after_launch();
+    const cudaError_t e = launch_chained(hex_apply_kernel, dim3(blocks_for(a.nslots)), kBlock, s, a);
+    return e != cudaSuccess ? e : after_launch();
 }
 
 cudaError_t launch_half_kick_back(const Arena& a, cudaStream_t s) {

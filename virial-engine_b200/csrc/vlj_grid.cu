@@ -80,12 +80,15 @@ __global__ void load_particles_kernel(Arena a) {
 // reorder_every-th rebuild (counted before the increment, as the reference).
 template <bool SET_CONDITION>
 __global__ void decide_kernel(Arena a, cudaGraphConditionalHandle handle) {
+    chain_wait();
     count_kernel(a);
     decide_block(a, handle, SET_CONDITION);
 }
 
 // ---- bin (grid.wgsl:11-38): cell of each slot from its f32 position ----
 __global__ void bin_kernel(Arena a) {
+    chain_next();
+    chain_wait();
     count_kernel(a);
     if (!grid_pass(a)) return;
     for_rebuild_slots(a, [&](uint32_t i, uint32_t b) {
@@ -134,6 +137,8 @@ constexpr uint32_t kScanChunk = (uint32_t)kScanThreads * kScanPer;
 __device__ __forceinline__ void scan_chunk(const Arena& a, const Box& bx, uint32_t tile);
 
 __global__ void __launch_bounds__(kScanThreads) scan_kernel(Arena a) {
+    chain_next();
+    chain_wait();
     count_kernel(a);
     if (!grid_pass(a)) return;
     const uint32_t boxes = a.glob->rb_boxes;
@@ -271,6 +276,8 @@ __device__ __forceinline__ void scan_chunk(const Arena& a, const Box& bx, uint32
 // ---- scatter (grid.wgsl:119-127): slot into its cell's last free place, the
 // cell's count running down to zero ----
 __global__ void scatter_kernel(Arena a) {
+    chain_next();
+    chain_wait();
     count_kernel(a);
     if (!grid_pass(a)) return;
     for_rebuild_slots(a, [&](uint32_t i, uint32_t) {
@@ -344,6 +351,8 @@ __device__ __forceinline__ void sort_big_cell(const Arena& a, uint32_t cell, uin
 }
 
 __global__ void __launch_bounds__(kBlock, 4) sort_kernel(Arena a) {
+    chain_next();
+    chain_wait();
     count_kernel(a);
     if (!grid_pass(a)) return;
     const uint32_t lane = threadIdx.x & 31u;
@@ -422,6 +431,8 @@ __global__ void __launch_bounds__(kBlock, 4) sort_kernel(Arena a) {
 
 // ---- reorder copy back (lennard_jones.wgsl:435-452) ----
 __global__ void reorder_kernel(Arena a) {
+    chain_next();
+    chain_wait();
     count_kernel(a);
     if (!a.glob->any) return;
     for_rebuild_slots(a, [&](uint32_t s, uint32_t b) {
@@ -459,28 +470,29 @@ cudaError_t launch_load_particles(const Arena& a, cudaStream_t s) {
 
 cudaError_t launch_decide(const Arena& a, cudaStream_t s, unsigned long long cond_handle) {
     const unsigned threads = a.nboxes == 1u ? 32u : 512u;  // a single box takes one thread
-    if (cond_handle)
-        decide_kernel<true><<<1, threads, 0, s>>>(a, (cudaGraphConditionalHandle)cond_handle);
-    else
-        decide_kernel<false><<<1, threads, 0, s>>>(a, (cudaGraphConditionalHandle)0);
-    return after_launch();
+    const cudaGraphConditionalHandle h = (cudaGraphConditionalHandle)cond_handle;
+    const cudaError_t e = launch_chained(cond_handle ? decide_kernel<true> : decide_kernel<false>, dim3(1),
+                                         threads, s, a, h);
+    return e != cudaSuccess ? e : after_launch();
 }
 
 cudaError_t launch_grid(const Arena& a, cudaStream_t s) {
     // the per-particle kernels cover the rebuilding boxes' particles from a
     // resident grid
     const unsigned slots = (unsigned)sm_count() * 8u;
-    bin_kernel<<<slots, kBlock, 0, s>>>(a);
+    cudaError_t e = launch_chained(bin_kernel, dim3(slots), kBlock, s, a);
     const dim3 scan(std::min(64u, (a.max_cells + kScanChunk - 1u) / kScanChunk), std::min(64u, a.nboxes));
-    scan_kernel<<<scan, kScanThreads, 0, s>>>(a);
-    scatter_kernel<<<slots, kBlock, 0, s>>>(a);
-    sort_kernel<<<(unsigned)sm_count() * 8u, kBlock, 0, s>>>(a);
+    if (e == cudaSuccess) e = launch_chained(scan_kernel, scan, kScanThreads, s, a);
+    if (e == cudaSuccess) e = launch_chained(scatter_kernel, dim3(slots), kBlock, s, a);
+    if (e == cudaSuccess) e = launch_chained(sort_kernel, dim3((unsigned)sm_count() * 8u), kBlock, s, a);
+    if (e != cudaSuccess) return e;
     return after_launch(4);
 }
 
 cudaError_t launch_lists(const Arena& a, cudaStream_t s) {
-    reorder_kernel<<<(unsigned)sm_count() * 8u, kBlock, 0, s>>>(a);
-    launch_build_list(a, s);  // vlj_build.cu
+    cudaError_t e = launch_chained(reorder_kernel, dim3((unsigned)sm_count() * 8u), kBlock, s, a);
+    if (e == cudaSuccess) e = launch_build_list(a, s);  // vlj_build.cu
+    if (e != cudaSuccess) return e;
     return after_launch(2);
 }
 
