@@ -51,7 +51,8 @@ __device__ __forceinline__ void df_parts(const double* pos, uint32_t i, float h[
 // which are not written).
 // One thread a grain spent its time on chains of dependent loads, a cell and
 // a candidate after the other: 67 us for 100,000 grains of a packed bed
-// (49 candidates a grain), 41 us so.
+// (49 candidates a grain), 41 us so. (A whole warp a grain: a pass of 98 us
+// against 90, its last lanes idle.)
 constexpr uint32_t kGrainLanes = 16;
 
 __global__ void __launch_bounds__(128) grain_contacts_kernel(const double* __restrict__ pos,
