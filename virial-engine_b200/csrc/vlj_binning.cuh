@@ -14,6 +14,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "vlj_place.h"
+
 namespace vlj {
 namespace {
 
@@ -117,15 +119,16 @@ __global__ void __launch_bounds__(1024) nb_scan(BinGrid g, uint32_t per, const u
 }
 
 // Each particle takes the last free place of its cell: the counts run down to
-// zero, so they need no pass that makes cursors of them.
+// zero, so they need no pass that makes cursors of them. The place, not the
+// counter, is checked (scatter_place).
 __global__ void nb_scatter(BinGrid g, const uint32_t* __restrict__ cell_of,
                            const uint32_t* __restrict__ cell_start, uint32_t* __restrict__ counts,
                            uint32_t* __restrict__ sorted) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= g.n) return;
     const uint32_t c = cell_of[i];
-    const uint32_t left = atomicSub(&counts[c], 1u);
-    if (left) sorted[cell_start[c] + left - 1u] = i;  // 0 only where two calls share a scratch
+    uint32_t at;
+    if (scatter_place(cell_start[c], atomicSub(&counts[c], 1u), g.n, &at)) sorted[at] = i;
 }
 
 // One warp per cell: each index's rank is the number of smaller indices in
@@ -203,7 +206,7 @@ __global__ void __launch_bounds__(kSortThreads) nb_order_large(const uint32_t* _
 inline cudaError_t enqueue_binning(const double* pos, const BinGrid& g, uint32_t* counts,
                                    uint32_t* sorted, uint32_t* cell_start, uint32_t* cell_of,
                                    cudaStream_t s) {
-    // the scratch keeps the previous call's cursors: counts start at zero
+    // the scratch keeps the previous call's list of crowded cells: counts start at zero
     cudaError_t e = cudaMemsetAsync(counts, 0, sizeof(uint32_t) * g.total, s);
     if (e != cudaSuccess) return e;
     const unsigned blocks = (g.n + 255u) / 256u;

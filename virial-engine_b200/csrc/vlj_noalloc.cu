@@ -21,10 +21,9 @@
 namespace vlj {
 namespace {
 
-// Per-cell counts, then fill cursors, shared by every call on a device; once
-// the particles are scattered, the same words list the cells of more than 32
-// particles for the block-wide sort, and the word after the last cell counts
-// them.
+// Per-cell counts, shared by every call on a device; the scatter runs them
+// down to zero, then the same words list the cells of more than 32 particles
+// for the block-wide sort, and the word after the last cell counts them.
 __device__ __align__(256) uint32_t g_bin_scratch[VLJ_BIN_NOALLOC_MAX_CELLS + 1];
 
 // The device address of the scratch array in the current device's context.
