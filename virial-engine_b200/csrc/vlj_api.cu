@@ -198,9 +198,10 @@ vlj_status upload_particles(vlj_sim* s, const vlj_particle* p, size_t count) {
 // The rebuild decision, and the rebuild where it is due, ahead of a pass over
 // the lists. Between two such passes with no step (and nothing else that
 // clears lists_current) nothing has moved and the second decision would find
-// nothing to do, so it is not launched.
+// nothing to do, so it is not launched -- unless some of the work lies in a
+// graph of the caller's, whose launches are not seen here.
 vlj_status lists_now(vlj_sim* s) {
-    if (s->lists_current) return VLJ_OK;
+    if (s->lists_current && !sim_note_capture(s)) return VLJ_OK;
     s->one_ready = false;
     if (s->use_graphs && !s->timing) {
         TRY(sim_launch_lists_graph(s));
@@ -1000,6 +1001,15 @@ vlj_status sim_settle(vlj_sim* s) {
 
 vlj_status sim_lists_now(vlj_sim* s) { return lists_now(s); }
 
+bool sim_note_capture(vlj_sim* s) {
+    if (!s->captured) {
+        cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(s->stream, &st) != cudaSuccess) cudaGetLastError();
+        s->captured = st != cudaStreamCaptureStatusNone;
+    }
+    return s->captured;
+}
+
 // Cell tiles for the step kernel of a single box (tile_step_kernel), when
 // VLJ_TILES=1 at creation: bricks of whole cells along x sized for about 112
 // home particles at the box's occupancy (its mean, or 0.9 particles per unit
@@ -1366,7 +1376,10 @@ static vlj_status step_direct(vlj_sim* s, bool heat = false) {
 }
 
 vlj_status sim_enqueue_steps(vlj_sim* s, uint32_t steps) {
-    if (steps > 0) s->lists_current = false;
+    if (steps > 0) {
+        sim_note_capture(s);
+        s->lists_current = false;
+    }
     if (steps > 0 && s->heat_pending) {
         // the first step's force pass takes the requested heat-current sample
         if (s->timing || !s->use_graphs) {

@@ -106,6 +106,9 @@ struct vlj_sim {
     bool one_ready = false;
     // the lists were brought up to date and nothing has changed since (lists_now)
     bool lists_current = false;
+    // some of the sim's work was enqueued while the caller captured its stream:
+    // from then on it may run again at any time, unseen by the host
+    bool captured = false;
     cudaGraphExec_t graph_one_heat = nullptr;  // one step that also takes the pending sample
     cudaGraphExec_t graph_lists = nullptr;  // decide -> IF(rebuild){rebuild chain}
     // per-launch timing of the step kernel (direct launches while on)
@@ -121,6 +124,8 @@ vlj_status sim_allocate(vlj_sim* s, void* stream);
 vlj_status make_list_map(const Arena& a, uint32_t rows, CUtensorMap* out);
 // Decide and, when due, rebuild the lists now (positions are about to be read).
 vlj_status sim_lists_now(vlj_sim* s);
+// Whether work was, or is being, captured into a graph of the caller's.
+bool sim_note_capture(vlj_sim* s);
 // Everything enqueued so far, then the status words, waited for; an error
 // where a kernel recorded a fault.
 vlj_status sim_read_status(vlj_sim* s);
