@@ -368,6 +368,9 @@ VLJ_API vlj_status vlj_debug_force_rebuild(vlj_sim *sim);
  * and the raw 64-bit fixed-point slots (8). */
 VLJ_API vlj_status vlj_debug_read_partials(vlj_sim *sim, float *pe_half, float *w_half,
                                            int64_t *raw_slots);
+/* Writes the word in which a kernel records a fault (0: none, 1: a wait that
+ * ran out), from the host, to test what the calls report; waits. */
+VLJ_API vlj_status vlj_debug_set_fault(vlj_sim *sim, uint32_t code);
 /* Kernel launches this library enqueued from the host so far (all
  * simulations; a graph launch counts its always-run nodes). */
 VLJ_API vlj_status vlj_debug_launches(uint64_t *launches);

@@ -282,6 +282,34 @@ vlj_status enqueue_measure(vlj_sim* s, int slot) {
     return VLJ_OK;
 }
 
+// The finished measurements, oldest first, and the fault word that came with
+// the newest of them.
+vlj_status poll_ring(vlj_sim* s, vlj_measurement* out, size_t capacity, size_t* written, uint32_t* fault) {
+    *written = 0;
+    *fault = 0;
+    std::vector<std::pair<uint64_t, int>> ready;
+    for (int k = 0; k < kRing; k++) {
+        if (!s->ring_busy[k]) continue;
+        cudaError_t e = cudaEventQuery(s->ring_event[k]);
+        if (e == cudaSuccess)
+            ready.push_back({s->ring_step[k], k});
+        else if (e != cudaErrorNotReady)
+            return fail(VLJ_CUDA_ERROR, "measurement read-back: %s", cudaGetErrorString(e));
+    }
+    std::sort(ready.begin(), ready.end());
+    size_t n = 0;
+    for (auto& r : ready) {
+        if (n >= capacity || !out) break;
+        out[n] = decode(s, s->ring[r.second], r.first);
+        if (out[n].list_overflow && s->list_growth) s->grow_pending = true;
+        *fault = s->ring[r.second].glob.fault;
+        n++;
+        s->ring_busy[r.second] = false;
+    }
+    *written = n;
+    return VLJ_OK;
+}
+
 }  // namespace
 
 vlj_sim::~vlj_sim() {
@@ -409,28 +437,8 @@ vlj_status vlj_measure(vlj_sim* s, int* accepted) {
 
 vlj_status vlj_poll(vlj_sim* s, vlj_measurement* out, size_t capacity, size_t* written) {
     if (!s || !written) return fail(VLJ_INVALID_ARG, "null argument");
-    *written = 0;
-    std::vector<std::pair<uint64_t, int>> ready;
-    for (int k = 0; k < kRing; k++) {
-        if (!s->ring_busy[k]) continue;
-        cudaError_t e = cudaEventQuery(s->ring_event[k]);
-        if (e == cudaSuccess)
-            ready.push_back({s->ring_step[k], k});
-        else if (e != cudaErrorNotReady)
-            return fail(VLJ_CUDA_ERROR, "measurement read-back: %s", cudaGetErrorString(e));
-    }
-    std::sort(ready.begin(), ready.end());
-    size_t n = 0;
-    for (auto& r : ready) {
-        if (n >= capacity || !out) break;
-        out[n] = decode(s, s->ring[r.second], r.first);
-        if (out[n].list_overflow && s->list_growth) s->grow_pending = true;
-        if (s->ring[r.second].glob.fault) s->polled_fault = s->ring[r.second].glob.fault;
-        n++;
-        s->ring_busy[r.second] = false;
-    }
-    *written = n;
-    return VLJ_OK;
+    uint32_t fault = 0;
+    return poll_ring(s, out, capacity, written, &fault);
 }
 
 vlj_status vlj_measure_now(vlj_sim* s, vlj_measurement* out) {
@@ -441,11 +449,10 @@ vlj_status vlj_measure_now(vlj_sim* s, vlj_measurement* out) {
     CUDA_TRY(cudaStreamSynchronize(s->stream));
     vlj_measurement buf[kRing];
     size_t n = 0;
-    TRY(vlj_poll(s, buf, kRing, &n));
+    uint32_t fault = 0;
+    TRY(poll_ring(s, buf, kRing, &n, &fault));
     if (n == 0) return fail(VLJ_CUDA_ERROR, "the measurement did not finish");
     *out = buf[n - 1];
-    const uint32_t fault = s->polled_fault;
-    s->polled_fault = 0;
     TRY(fault_status(fault));
     if (out->list_overflow && s->list_growth) {
         // lists that dropped pairs: grow them, rebuild, measure again
@@ -700,6 +707,13 @@ vlj_status vlj_debug_force_rebuild(vlj_sim* s) {
                              s->stream));
     s->lists_current = false;
     TRY(lists_now(s));
+    CUDA_TRY(cudaStreamSynchronize(s->stream));
+    return VLJ_OK;
+}
+
+vlj_status vlj_debug_set_fault(vlj_sim* s, uint32_t code) {
+    if (!s) return fail(VLJ_INVALID_ARG, "sim is null");
+    CUDA_TRY(cudaMemcpyAsync(&s->arena.glob->fault, &code, sizeof code, cudaMemcpyHostToDevice, s->stream));
     CUDA_TRY(cudaStreamSynchronize(s->stream));
     return VLJ_OK;
 }

@@ -64,11 +64,9 @@ struct vlj_sim {
     cudaEvent_t ring_event[vlj::kRing] = {};
     bool ring_busy[vlj::kRing] = {};
     uint64_t ring_step[vlj::kRing] = {};
-    // those words of every box, pinned (sim_read_status), and a fault that a
-    // polled measurement came with
+    // those words of every box, pinned (sim_read_status)
     unsigned char* status = nullptr;
     size_t status_bytes = 0;
-    uint32_t polled_fault = 0;
     const long long* status_slots() const { return reinterpret_cast<const long long*>(status); }
     const vlj::Control* status_ctrl() const {
         return reinterpret_cast<const vlj::Control*>(status + sizeof(long long) * vlj::kSlots * arena.nboxes);

@@ -567,6 +567,10 @@ class LennardJones:
     def force_rebuild(self):
         _check(_lib.vlj_debug_force_rebuild(self._h))
 
+    def set_fault(self, code):
+        """The word in which a kernel records a fault, written from the host."""
+        _check(_lib.vlj_debug_set_fault(self._h, int(code)))
+
     def read_partials(self):
         """(pe, w, raw): per-slot (hi, lo) halves of pair energy and virial."""
         pe = np.zeros((self._n, 2), np.float32)

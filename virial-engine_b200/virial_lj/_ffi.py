@@ -113,6 +113,7 @@ SIGNATURES = {
     "vlj_debug_grid_info": [_vp, _P(GridInfo)],
     "vlj_debug_read_grid": [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp],
     "vlj_debug_force_rebuild": [_vp],
+    "vlj_debug_set_fault": [_vp, C.c_uint32],
     "vlj_debug_read_partials": [_vp, _vp, _vp, _vp],
     "vlj_debug_launches": [_P(C.c_uint64)],
     "vlj_debug_kernels_executed": [_vp, _P(C.c_uint64)],
