@@ -316,7 +316,7 @@ def run_batched(args, world, rank, stream, flush_l2, hbm_peak, fp32_peak):
             sim = vl.LennardJones(r.particles, st, stream=stream.cuda_stream)
         except vl.VljError:
             continue  # a box under three cells wide: the plain path refuses it
-        sim.step(3)
+        sim.step(PLAIN_SAMPLE_STEPS)  # captures the graphs that these steps take
         e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
         stream.synchronize()
         e0.record(stream)
@@ -382,7 +382,9 @@ def run_slab(args, world, rank, stream, flush_l2):
                                          thermostat=vl.Langevin(SLAB["temperature"],
                                                                 SLAB["friction"], 11 + rank)),
                           stream=stream.cuda_stream)
-    sim.step(max(args.warmup, 3) * SLAB["every"])
+    # warmed in the calls that are timed; the 32nd captures the graph of their last four steps
+    for _ in range(max(args.warmup, 33)):
+        sim.step(SLAB["every"])
     sim.clear_profile()
     cycles = max(args.steps // SLAB["every"], 5)
     ev = [(torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True))
@@ -444,7 +446,7 @@ def run_small(args, world, rank, stream, flush_l2):
     sim.step(50)  # warm-up on a copy, to build the graphs
     sim.close()
     sim = vl.LennardJones(p, st, stream=stream.cuda_stream)
-    sim.step(16)
+    sim.step(17)  # a graph of 16 steps and one of a single step, which the run takes
     m0 = sim.measure_now()
     stream.synchronize()
     barrier(world)

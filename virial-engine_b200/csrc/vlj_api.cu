@@ -313,8 +313,8 @@ vlj_status poll_ring(vlj_sim* s, vlj_measurement* out, size_t capacity, size_t* 
 }  // namespace
 
 vlj_sim::~vlj_sim() {
-    for (cudaGraphExec_t g : graph_chunk)
-        if (g) cudaGraphExecDestroy(g);
+    if (graph_chunk) cudaGraphExecDestroy(graph_chunk);
+    if (graph_short) cudaGraphExecDestroy(graph_short);
     if (graph_one) cudaGraphExecDestroy(graph_one);
     if (graph_one_tmpl) cudaGraphDestroy(graph_one_tmpl);
     if (graph_one_heat) cudaGraphExecDestroy(graph_one_heat);
@@ -413,7 +413,7 @@ vlj_status vlj_step(vlj_sim* s, uint32_t steps) {
 vlj_status vlj_run(vlj_sim* s, uint64_t steps) {
     if (!s) return fail(VLJ_INVALID_ARG, "sim is null");
     while (steps > 0) {
-        uint32_t batch = (uint32_t)std::min<uint64_t>(steps, 200);
+        uint32_t batch = (uint32_t)std::min<uint64_t>(steps, kRunSteps);
         TRY(vlj_step(s, batch));
         steps -= batch;
     }
@@ -1410,16 +1410,25 @@ vlj_status sim_enqueue_steps(vlj_sim* s, uint32_t steps) {
         for (uint32_t k = 0; k < steps; k++) TRY(step_direct(s));
         return VLJ_OK;
     }
-    // Whole graphs of 16, then one each of 8, 4 and 2, then a single step: a
-    // graph launch more costs about 5 us (four steps of 32,768 atoms and a read-out: 290 us
-    // as four launches, 273 as one).
-    for (int k = 0; k < kChunks; k++) {
-        const uint32_t count = kGraphChunk >> k;
-        for (; steps >= count; steps -= count) {
-            if (!s->graph_chunk[k]) TRY(build_graph(s, count, &s->graph_chunk[k]));
-            CUDA_TRY(cudaGraphLaunch(s->graph_chunk[k], s->stream));
-            s->one_ready = false;  // the chunk's last step leaves the decision open
-        }
+    // Whole graphs of 16 steps, then, once captured, of 4, then single steps.
+    // At 1,000 atoms a graph of 4 saves about 8 us over its steps one by one
+    // (a run of 4 steps: 72 us against 80, of 31: 610 against 625), but
+    // capturing costs about 65 us a step of the graph. So the graphs of 16 and
+    // of one step are captured when first needed, and the one of 4 in the call
+    // by which it would have saved its price: a short-lived simulation, or one
+    // whose calls are of ever new lengths, captures 17 steps at most. (With
+    // graphs of 8 and 2 beside it, all captured when first needed, a first run
+    // of 31 steps took 2,780 us, 1,900 so; those two saved less than 3 us a call.)
+    for (; steps >= kGraphChunk; steps -= kGraphChunk) {
+        if (!s->graph_chunk) TRY(build_graph(s, kGraphChunk, &s->graph_chunk));
+        CUDA_TRY(cudaGraphLaunch(s->graph_chunk, s->stream));
+        s->one_ready = false;  // the chunk's last step leaves the decision open
+    }
+    if (steps >= kGraphShort && !s->graph_short && ++s->short_uses >= kShortUses)
+        TRY(build_graph(s, kGraphShort, &s->graph_short));
+    for (; steps >= kGraphShort && s->graph_short; steps -= kGraphShort) {
+        CUDA_TRY(cudaGraphLaunch(s->graph_short, s->stream));
+        s->one_ready = false;
     }
     if (steps > 0 && !s->graph_one) {
         s->one_decide = nullptr;
@@ -1534,17 +1543,16 @@ vlj_status sim_grow_lists(vlj_sim* s, bool* grew) {
 }
 
 void sim_drop_step_graphs(vlj_sim* s) {
-    for (cudaGraphExec_t& g : s->graph_chunk) {
-        if (g) cudaGraphExecDestroy(g);
-        g = nullptr;
-    }
+    if (s->graph_chunk) cudaGraphExecDestroy(s->graph_chunk);
+    if (s->graph_short) cudaGraphExecDestroy(s->graph_short);
+    s->short_uses = 0;
     if (s->graph_one) cudaGraphExecDestroy(s->graph_one);
     if (s->graph_one_tmpl) cudaGraphDestroy(s->graph_one_tmpl);
     s->graph_one_tmpl = nullptr;
     s->one_decide = nullptr;
     s->one_ready = false;
     if (s->graph_one_heat) cudaGraphExecDestroy(s->graph_one_heat);
-    s->graph_one = s->graph_one_heat = nullptr;
+    s->graph_chunk = s->graph_short = s->graph_one = s->graph_one_heat = nullptr;
 }
 
 }  // namespace vlj

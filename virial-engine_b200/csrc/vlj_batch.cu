@@ -218,7 +218,7 @@ vlj_status vlj_batch_step(vlj_batch* bt, uint32_t steps) {
 vlj_status vlj_batch_run(vlj_batch* bt, uint64_t steps) {
     if (!bt) return fail(VLJ_INVALID_ARG, "batch is null");
     while (steps > 0) {
-        const uint32_t chunk = (uint32_t)std::min<uint64_t>(steps, 200);
+        const uint32_t chunk = (uint32_t)std::min<uint64_t>(steps, kRunSteps);
         TRY(vlj_batch_step(bt, chunk));
         steps -= chunk;
     }

@@ -14,7 +14,12 @@ namespace vlj {
 
 constexpr int kRing = 3;  // measurement read-back slots (lennard_jones.rs:320)
 constexpr uint32_t kGraphChunk = 16;  // most steps per graph launch
-constexpr int kChunks = 4;            // graphs of 16, 8, 4 and 2 steps
+constexpr uint32_t kGraphShort = 4;   // steps of the graph that takes what is left of a call
+// The call with such a rest in which that graph is captured (sim_enqueue_steps);
+// until then its steps go out one by one.
+constexpr uint32_t kShortUses = 32;
+// Steps that a run enqueues at a time: whole graphs of 16.
+constexpr uint32_t kRunSteps = 12 * kGraphChunk;
 
 // The words the host reads back, one after the other on the device (the
 // measurement sums, control words and thermostats of every box, then the
@@ -88,12 +93,14 @@ struct vlj_sim {
     double* pin_x = nullptr;
     double* pin_v = nullptr;
     uint32_t* pin_id = nullptr;
-    // captured steps: graphs of kGraphChunk >> k steps and one of a single
-    // step, each captured when first needed, each step's rebuild chain under
-    // a conditional node
+    // captured steps: graphs of kGraphChunk, kGraphShort and one steps, each
+    // step's rebuild chain under a conditional node; the short one is captured
+    // in the kShortUses-th call with a use for it, the others when first needed
     bool use_graphs = true;
     cudaStream_t capture_stream = nullptr;
-    cudaGraphExec_t graph_chunk[vlj::kChunks] = {};
+    cudaGraphExec_t graph_chunk = nullptr;
+    cudaGraphExec_t graph_short = nullptr;
+    uint32_t short_uses = 0;  // calls with a use for it since the graphs were last dropped
     cudaGraphExec_t graph_one = nullptr;
     // graph_one's template (kept for node updates) and its decide node: while
     // the last step enqueued was graph_one's, whose step kernel took this

@@ -768,8 +768,9 @@ def tune_batch(replicas, skins=(0.3, 0.4, 0.5, 0.6, 0.8), threads=(64, 128, 256)
     The skin trades list length against rebuild frequency (tune_batch_skin);
     the block size trades the step kernel's tail (blocks that straddle two
     replicas, or hold a dense replica's long lists) against its scheduling
-    granularity. Every (skin, threads) pair runs `warmup` then `steps` steps
-    of the actual set, timed with CUDA events on `stream` (a torch stream);
+    granularity. Every skin runs `warmup` steps of the actual set, then every
+    block size `steps` untimed and `steps` timed ones, with CUDA events on
+    `stream` (a torch stream);
     the trajectory does not depend on the block size and only the list length
     on the skin. Returns (skin, threads, {(skin, threads): seconds per step}).
     """
@@ -783,7 +784,7 @@ def tune_batch(replicas, skins=(0.3, 0.4, 0.5, 0.6, 0.8), threads=(64, 128, 256)
         b.step(warmup)
         for t in threads:
             b.set_step_threads(t)
-            b.step(3)
+            b.step(steps)  # untimed: captures the graphs that these steps take
             e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
             e0.record(s)
             b.step(steps)
@@ -854,9 +855,9 @@ def tune_batch_skin(replicas, skins=(0.3, 0.4, 0.5, 0.6, 0.8), cutoff=2.5, dt=0.
 
     A wider skin makes longer lists (more work every step) but rebuilds them
     less often; the best trade depends on the replicas' densities and
-    temperatures, so each candidate runs `warmup` then `steps` steps of the
-    actual set (timed with CUDA events through `torch.cuda`, on `stream`, a
-    torch stream). Forces are exact within the cutoff at any skin, so the choice
+    temperatures, so each candidate runs `warmup` and `steps` untimed, then
+    `steps` timed steps of the actual set (CUDA events through `torch.cuda`, on
+    `stream`, a torch stream). Forces are exact within the cutoff at any skin, so the choice
     changes speed, not physics. Returns (best skin, {skin: seconds per step}).
     """
     import torch
@@ -867,6 +868,7 @@ def tune_batch_skin(replicas, skins=(0.3, 0.4, 0.5, 0.6, 0.8), cutoff=2.5, dt=0.
         b = Batch(replicas, cutoff=cutoff, skin=skin, dt=dt, shifted_force=shifted_force,
                   stream=s.cuda_stream)
         b.step(warmup)
+        b.step(steps)  # untimed: captures the graphs that these steps take
         e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
         e0.record(s)
         b.step(steps)
