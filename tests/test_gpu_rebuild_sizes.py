@@ -18,6 +18,7 @@ CASES = {
     # and more chunks than the grid has blocks
     "one_chunk": (3000, [44.9] * 3), "one_chunk_and_a_row": (3000, [44.9, 44.9, 47.7]),
     "chunks_dilute": (30000, [70.1, 84.1, 98.1]), "chunks_again": (25000, [182.1] * 3),
+    "chunks_most": (25000, [283.5] * 3),
 }
 
 
@@ -33,3 +34,21 @@ def test_rebuild_at_the_edges_of_its_launches(gpu, O, case):
         sim.force_rebuild()
         compare_rebuild(sim, O, dict(x=pre["x"], v=pre["v"], ids=pre["ids"]), before % 4 == 0)
     sim.close()
+
+
+def test_scan_of_more_cells_than_some_waves_of_blocks(gpu):
+    # six boxes of 1,030,301 cells each: blocks take runs of chunks that a box
+    # by itself would not; the same trajectories as the boxes by themselves
+    box = [283.5] * 3
+    parts = [gpu.lattice_box(1500 + 7 * r, box, 1.2, r) for r in range(6)]
+    batch = gpu.Batch([gpu.Replica(p, box, None) for p in parts], dt=0.005)
+    batch.run(37)
+    got = [batch.read_particles(r) for r in range(6)]
+    rebuilds = [m.list_rebuilds for m in batch.measure()]
+    batch.close()
+    for p, q, n in zip(parts, got, rebuilds):
+        sim = gpu.LennardJones(p, gpu.Settings(box, dt=0.005))
+        sim.run(37)
+        assert sim.read_particles().tobytes() == q.tobytes()
+        assert sim.measure_now().list_rebuilds == n > 2
+        sim.close()

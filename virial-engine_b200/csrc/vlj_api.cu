@@ -1096,6 +1096,7 @@ vlj_status sim_allocate(vlj_sim* s, void* stream) {
         slots += b.n;
         cells += b.total_cells;
         a.max_cells = std::max(a.max_cells, b.total_cells);
+        a.scan_chunks += (b.total_cells + kScanChunk - 1u) / kScanChunk;
         cap = std::max(cap, b.capacity);
     }
     if (slots >= (1ull << 30)) return fail(VLJ_INVALID_ARG, "at most 2^30 - 1 particles in all");

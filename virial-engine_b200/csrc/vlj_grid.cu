@@ -8,10 +8,10 @@
 // once when nothing rebuilds. Reference kernels are cited at each kernel.
 #include <cuda_runtime.h>
 
-#include <algorithm>
 #include <atomic>
 
 #include "vlj_device.cuh"
+#include "vlj_scan_shape.h"
 #include "vlj_internal.cuh"
 
 namespace vlj {
@@ -116,13 +116,16 @@ __global__ void bin_kernel(Arena a) {
 }
 
 // ---- scan (grid.wgsl:43-117): exclusive prefix sum of a box's counts
-// offset by its first slot, a block per kScanChunk cells (the grid's y strides
-// through the rebuilding boxes). A block first adds up the counts of the box's
-// cells before its own -- a few loads a thread, against a pass after the
-// other in one block: with one block a box the shuffles of 32 warps on one SM
-// were the time (11 us for a box of 12,167 cells, 84 us for 117,649; 6.6
-// and 11.9 us so). The counts stay as they are: the scatter runs them down
-// to zero.
+// offset by its first slot, a block per run of chunks of kScanChunk cells (the
+// grid's y strides through the rebuilding boxes). A block first adds up the
+// counts of the box's cells before its run -- a few loads a thread, against a
+// pass after the other in one block: with one block a box the shuffles of 32
+// warps on one SM were the time (11 us for a box of 12,167 cells, 84 us for
+// 117,649; 6.6 and 11.9 us so). A run is one chunk in all but very large
+// boxes or sets of them (scan_shape): 128 boxes of 2^20 dilute cells take 201 us
+// a step on average, rebuilds among them, against 546 with single chunks and
+// 296 with a block a box; 400 of them 462, 1,512 and 451. The counts stay as
+// they are: the scatter runs them down to zero.
 // The box's non-empty cells join the step's work list for the sort and the
 // list build as entries cell * 8 + part: cells of kDenseCell particles or
 // more at its front, the others at its back; where cells split (part_homes)
@@ -132,11 +135,11 @@ __global__ void bin_kernel(Arena a) {
 // totals, and one atomic per block and class reserves its work-list entries.
 constexpr int kScanThreads = 1024;
 constexpr int kScanPer = 4;  // runs of 32 cells per warp
-constexpr uint32_t kScanChunk = (uint32_t)kScanThreads * kScanPer;
+static_assert(kScanChunk == (uint32_t)kScanThreads * kScanPer, "a chunk is one pass of a block");
 
-__device__ __forceinline__ void scan_chunk(const Arena& a, const Box& bx, uint32_t tile);
+__device__ __forceinline__ uint32_t scan_chunk(const Arena& a, const Box& bx, uint32_t tile, uint32_t t);
 
-__global__ void __launch_bounds__(kScanThreads) scan_kernel(Arena a) {
+__global__ void __launch_bounds__(kScanThreads) scan_kernel(Arena a, uint32_t least) {
     chain_next();
     chain_wait();
     count_kernel(a);
@@ -144,12 +147,22 @@ __global__ void __launch_bounds__(kScanThreads) scan_kernel(Arena a) {
     const uint32_t boxes = a.glob->rb_boxes;
     for (uint32_t k = blockIdx.y; k < boxes; k += gridDim.y) {
         const Box& bx = a.boxes[a.rb_box[k]];
-        for (uint32_t tile = blockIdx.x * kScanChunk; tile < bx.total_cells; tile += gridDim.x * kScanChunk)
-            scan_chunk(a, bx, tile);
+        const uint32_t chunks = (bx.total_cells + kScanChunk - 1u) / kScanChunk;
+        const uint32_t run = scan_run(chunks, gridDim.x, least);
+        const uint32_t from = blockIdx.x * run;
+        if (from >= chunks) continue;
+        // this thread's share of the particles in the cells before the run
+        uint32_t t = 0;
+#pragma unroll 8
+        for (uint32_t c = threadIdx.x; c < from * kScanChunk; c += kScanThreads) t += a.count[bx.cell_base + c];
+        for (uint32_t chunk = from; chunk < min(chunks, from + run); chunk++)
+            t = scan_chunk(a, bx, chunk * kScanChunk, t);
     }
 }
 
-__device__ __forceinline__ void scan_chunk(const Arena& a, const Box& bx, uint32_t tile) {
+// One chunk, from cell `tile` of the box. The t of all threads add up to the
+// particles in the cells before it; returns the same for the next chunk.
+__device__ __forceinline__ uint32_t scan_chunk(const Arena& a, const Box& bx, uint32_t tile, uint32_t t) {
     __shared__ uint32_t s_sum[kScanThreads / 32], s_nd[kScanThreads / 32], s_ns[kScanThreads / 32];
     __shared__ uint32_t s_before[kScanThreads / 32];
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
@@ -157,12 +170,8 @@ __device__ __forceinline__ void scan_chunk(const Arena& a, const Box& bx, uint32
     const uint32_t total = bx.total_cells, base = bx.cell_base;
     const uint32_t per = part_homes(a, narrow_box(bx));
     {
-        // the box's particles in the cells before this chunk
-        uint32_t t = 0;
-#pragma unroll 8
-        for (uint32_t c = threadIdx.x; c < tile; c += kScanThreads) t += a.count[base + c];
-        t = __reduce_add_sync(0xffffffffu, t);
-        if (lane == 0) s_before[warp] = t;
+        const uint32_t before_warp = __reduce_add_sync(0xffffffffu, t);
+        if (lane == 0) s_before[warp] = before_warp;
         const uint32_t first = tile + warp * 32u * (uint32_t)kScanPer;
         uint32_t excl[kScanPer];  // within the warp's cells, before this lane's
         // nibble r: front entries of this lane's cell of run r (its parts,
@@ -179,6 +188,7 @@ __device__ __forceinline__ void scan_chunk(const Arena& a, const Box& bx, uint32
         for (int r = 0; r < kScanPer; r++) {
             const uint32_t c = first + 32u * (uint32_t)r + lane;
             excl[r] = c < total ? a.count[base + c] : 0u;
+            t += excl[r];
         }
 #pragma unroll
         for (int r = 0; r < kScanPer; r++) {
@@ -271,6 +281,7 @@ __device__ __forceinline__ void scan_chunk(const Arena& a, const Box& bx, uint32
         }
         __syncthreads();
     }
+    return t;
 }
 
 // ---- scatter (grid.wgsl:119-127): slot into its cell's last free place, the
@@ -495,8 +506,10 @@ cudaError_t launch_grid(const Arena& a, cudaStream_t s) {
     // resident grid
     const unsigned slots = (unsigned)sm_count() * 8u;
     cudaError_t e = launch_chained(bin_kernel, dim3(slots), kBlock, s, a);
-    const dim3 scan(std::min(64u, (a.max_cells + kScanChunk - 1u) / kScanChunk), std::min(64u, a.nboxes));
-    if (e == cudaSuccess) e = launch_chained(scan_kernel, scan, kScanThreads, s, a);
+    const ScanShape shape = scan_shape(a.scan_chunks, (a.max_cells + kScanChunk - 1u) / kScanChunk, a.nboxes,
+                                       (unsigned)sm_count());
+    const dim3 scan(shape.x, shape.y);
+    if (e == cudaSuccess) e = launch_chained(scan_kernel, scan, kScanThreads, s, a, shape.least);
     if (e == cudaSuccess) e = launch_chained(scatter_kernel, dim3(slots), kBlock, s, a);
     if (e == cudaSuccess) e = launch_chained(sort_kernel, dim3((unsigned)sm_count() * 8u), kBlock, s, a);
     if (e != cudaSuccess) return e;

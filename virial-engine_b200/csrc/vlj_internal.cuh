@@ -100,6 +100,7 @@ constexpr uint32_t kPartHomes = VLJ_PART_HOMES;
 #endif
 constexpr uint32_t kSplitSlots = VLJ_SPLIT_SLOTS;
 constexpr uint32_t kMaxParts = 8;
+constexpr uint32_t kScanChunk = 4096;  // cells of one pass of a block of the cell scan
 constexpr int kTileRows = VLJ_TILE_ROWS;
 constexpr int kTileSlots = VLJ_TILE_SLOTS;  // tiles in flight per block
 // measurement slots: 0 kinetic, 1 potential, 2 virial, 3-5 momentum,
@@ -229,6 +230,7 @@ struct Arena {
     uint32_t seg;        // padded slot count (list row length)
     uint32_t ncells;     // cells in all boxes
     uint32_t max_cells;  // cells of the box with the most
+    uint32_t scan_chunks;  // all boxes' cells in chunks of kScanChunk, each box's rounded up
     const uint32_t* box_of_slot;  // null for a single box
     const uint32_t* box_of_cell;  // null for a single box
     double* x;
