@@ -1164,7 +1164,8 @@ vlj_status sim_allocate(vlj_sim* s, void* stream) {
             const bool narrow = b.cells[0] < 5u || b.cells[1] < 5u || b.cells[2] < 5u;
             cap += (size_t)b.total_cells * (narrow ? kMaxParts : 1u);
         }
-        cap = std::max(cap, (size_t)std::min(n, kSplitSlots));
+        a.part_entries = std::max(1u, VLJ_PART_ENTRIES * (uint32_t)sm_count() / 148u);
+        cap = std::max(cap, (size_t)std::min(n, kPartHomes * a.part_entries));
         if (cap >= (1ull << 32)) return fail(VLJ_INVALID_ARG, "too many cells in all boxes");
         a.work_cap = (uint32_t)cap;
         TRY(dalloc(s, &a.work, cap));

@@ -15,7 +15,6 @@ inline unsigned blocks_for(uint64_t n, int threads = kBlock) {
 cudaError_t after_launch(unsigned n = 1);
 // Streaming multiprocessors of the current device (cached per device): the
 // grid of the kernels that loop over the step's work list.
-int sm_count();
 cudaError_t launch_build_list(const Arena& a, cudaStream_t s);  // vlj_build.cu
 
 // Chained launches: a kernel launched with launch_chained may start while the
@@ -82,14 +81,15 @@ __device__ __forceinline__ bool narrow_box(const Box& bx) {
 // A warp that builds a whole cell's lists is a chain of some 11,700
 // instructions, 46 us when it runs alone; with few particles to rebuild most
 // of the resident warps would have no cell, so the cells split until the
-// entries are about as many as those warps (some 3,500 on 148 SMs; a second
-// wave costs more than a longer part, and parts round up, hence the 2,400).
+// entries are about as many as those warps (3,552 on 148 SMs; a second wave
+// costs more than a longer part, and parts round up, hence the 2,400 there;
+// Arena::part_entries, in proportion to the SMs).
 // Every part stages the cell's candidates again, so no further than two
 // homes, and not at all where the cells fill the warps by themselves.
 __device__ __forceinline__ uint32_t part_homes(const Arena& a, bool narrow) {
     const uint32_t slots = a.glob->rb_slots;
-    if (slots > kSplitSlots) return narrow ? kPartHomes : 0u;
-    return min(kPartHomes, max(2u, (slots + 2399u) / 2400u));
+    if (slots > kPartHomes * a.part_entries) return narrow ? kPartHomes : 0u;
+    return min(kPartHomes, max(2u, (slots + a.part_entries - 1u) / a.part_entries));
 }
 
 // Work-list entries of a cell of m particles, split by `per` homes.

@@ -89,16 +89,16 @@ constexpr uint32_t kDenseCell = 8;  // particles in a cell the list build takes 
 // batched replica) a cell holds many particles and its candidate stream is
 // most of the box, so its home particles split into parts of about kPartHomes
 // (at most kMaxParts). Where the boxes that rebuild hold no more particles
-// than kSplitSlots, every cell splits, into parts small enough that the
-// entries fill the build's resident warps (part_homes).
+// than kPartHomes for each of Arena::part_entries, every cell splits, into
+// parts small enough that the entries fill the build's resident warps
+// (part_homes).
 #ifndef VLJ_PART_HOMES
 #define VLJ_PART_HOMES 8
 #endif
 constexpr uint32_t kPartHomes = VLJ_PART_HOMES;
-#ifndef VLJ_SPLIT_SLOTS
-#define VLJ_SPLIT_SLOTS 19200
+#ifndef VLJ_PART_ENTRIES
+#define VLJ_PART_ENTRIES 2400  // on 148 SMs
 #endif
-constexpr uint32_t kSplitSlots = VLJ_SPLIT_SLOTS;
 constexpr uint32_t kMaxParts = 8;
 constexpr uint32_t kScanChunk = 4096;  // cells of one pass of a block of the cell scan
 constexpr int kTileRows = VLJ_TILE_ROWS;
@@ -230,6 +230,7 @@ struct Arena {
     uint32_t seg;        // padded slot count (list row length)
     uint32_t ncells;     // cells in all boxes
     uint32_t max_cells;  // cells of the box with the most
+    uint32_t part_entries;  // work entries that split cells come to (part_homes)
     uint32_t scan_chunks;  // all boxes' cells in chunks of kScanChunk, each box's rounded up
     const uint32_t* box_of_slot;  // null for a single box
     const uint32_t* box_of_cell;  // null for a single box
@@ -477,6 +478,7 @@ __device__ __forceinline__ float encoded_r2(uint4 a, uint4 b, const float dec[3]
 }
 
 // ---- launchers (vlj_kernels.cu); every kernel takes the Arena by value ----
+int sm_count();
 cudaError_t launch_encode(const Arena& a, cudaStream_t s);
 // Particles from a.aos (input order) into the state of a single box: positions
 // wrapped into the box, ids the input order; a non-finite coordinate records
