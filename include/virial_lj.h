@@ -405,11 +405,12 @@ VLJ_API vlj_status vlj_debug_set_tiles(vlj_sim *sim, int on);
  * tuning knob: virial_lj.tune_batch times it per replica set; the same
  * trajectory to the bit). */
 VLJ_API vlj_status vlj_debug_set_step_threads(vlj_sim *sim, uint32_t threads);
-/* Lanes per particle of the step kernel: 0 (the default) chooses by grid
- * size (up to eight for small boxes), 1 or 2 forces one form. Every kernel
- * sums a particle's force in parts of two list rows, added in list order, so
- * the trajectory is the same to the bit either way; the switch is for tests
- * and timing. */
+/* Lanes per particle of the force passes (steps of every ensemble,
+ * measurements, particles out): 0 (the default) chooses by grid size (up to
+ * eight for small boxes), 1, 2, 4 or 8 forces one form. Every kernel sums a
+ * particle's force and energies in parts of two list rows, added in list order,
+ * so the results are the same to the bit either way; the switch is for tests
+ * and timing. A pass that takes a heat-current sample has one lane. */
 VLJ_API vlj_status vlj_debug_set_step_lanes(vlj_sim *sim, uint32_t lanes);
 VLJ_API vlj_status vlj_debug_tile_info(vlj_sim *sim, uint32_t *brick_cols, uint32_t *bricks,
                                        uint32_t *tile_cap, uint32_t *threads);
@@ -422,8 +423,8 @@ VLJ_API vlj_status vlj_debug_read_tile_lists(vlj_sim *sim, uint16_t *out);
 VLJ_API vlj_status vlj_debug_philox(const uint32_t *ctr, const uint32_t *key, size_t n,
                                     uint32_t *out, float *noise);
 /* The simulation that steps a batch's arena, for vlj_debug_set_graphs,
- * vlj_debug_kernel_timing / _time and vlj_debug_kernels_executed only (it
- * stays owned by the batch). */
+ * vlj_debug_set_step_threads / _lanes, vlj_debug_kernel_timing / _time and
+ * vlj_debug_kernels_executed only (it stays owned by the batch). */
 VLJ_API vlj_status vlj_debug_batch_sim(vlj_batch *batch, vlj_sim **sim);
 
 #ifdef __cplusplus

@@ -27,8 +27,10 @@ def test_rebuild_at_the_edges_of_its_launches(gpu, O, case):
     n, box = CASES[case]
     p = gpu.lattice_box(n, box, 1.3, 6)
     sim = gpu.LennardJones(p, gpu.Settings(box, dt=0.005, thermostat=gpu.Langevin(1.3, 1.0, 6)))
-    for _ in range(2):
-        sim.run(46)  # whole graphs: no decision left over from a single step
+    # 48 steps are whole graphs; of 45 the last ones run one by one and leave
+    # their decision for the next step, to which a forced rebuild adds
+    for steps in (48, 45):
+        sim.run(steps)
         pre = sim.read_grid()
         before = sim.grid_info().rebuilds
         sim.force_rebuild()

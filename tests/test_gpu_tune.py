@@ -108,9 +108,9 @@ def lanes_run(gpu, p, st, lanes, steps, heat_every=0):
 
 @pytest.mark.parametrize("case", ["lattice1000", "fcc20_langevin", "fcc40_langevin"])
 def test_two_lanes_per_particle_keep_the_trajectory(gpu, case):
-    # forces summed in two parts (even and odd list rows) in every kernel:
-    # two lanes a particle and one give the same bits, on a small box (where
-    # two lanes are the default), a mid-size and the 256k box
+    # forces summed in parts of two list rows in every kernel: two lanes a
+    # particle, one and those of the box's size give the same bits, on a small
+    # box (eight by its size), a mid-size one (two) and the 256k box (one)
     if case == "lattice1000":
         L = (1000 / 0.8442) ** (1 / 3)
         p = gpu.lattice(1000, L, 0.72, 1)

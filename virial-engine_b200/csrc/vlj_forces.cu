@@ -1362,6 +1362,9 @@ static int lanes_for(uint32_t n) {
     return 1;
 }
 
+// The same, unless a test asks for a number of lanes.
+static int lanes_of(const Arena& a, uint32_t n) { return a.step_lanes ? (int)a.step_lanes : lanes_for(n); }
+
 template <bool SF, int LANES, int THREADS>
 static void launch_lanes(const Arena& a, cudaStream_t s, cudaGraphConditionalHandle next) {
     static bool carved = false;
@@ -1393,7 +1396,7 @@ static cudaError_t launch_step_kernel(const Arena& a, const CUtensorMap& map, bo
         prefer_l1(step_kernel<false, true, THREADS>);
     }
 #if VLJ_LIST_STREAM
-    const int lanes = heat ? 1 : (a.step_lanes ? (int)a.step_lanes : lanes_for(a.nslots));
+    const int lanes = heat ? 1 : lanes_of(a, a.nslots);
     if (lanes > 1) {
         if (shifted_force) launch_step_lanes<true, THREADS>(a, lanes, s, next);
         else launch_step_lanes<false, THREADS>(a, lanes, s, next);
@@ -1472,7 +1475,7 @@ static void measure_lanes(const Arena& a, const CUtensorMap& map, cudaStream_t s
 template <bool SF>
 static void measure(const Arena& a, const CUtensorMap& map, cudaStream_t s) {
 #if VLJ_LIST_STREAM
-    switch (lanes_for(a.nslots)) {
+    switch (lanes_of(a, a.nslots)) {
         case 8: return measure_lanes<SF, 8>(a, map, s);
         case 4: return measure_lanes<SF, 4>(a, map, s);
         case 2: return measure_lanes<SF, 2>(a, map, s);
@@ -1505,7 +1508,7 @@ template <bool SF>
 static void read(const Arena& a, const CUtensorMap& map, uint32_t first, uint32_t count, double* out,
                  cudaStream_t s) {
 #if VLJ_LIST_STREAM
-    switch (lanes_for(count)) {
+    switch (lanes_of(a, count)) {
         case 8: return read_lanes<SF, 8>(a, map, first, count, out, s);
         case 4: return read_lanes<SF, 4>(a, map, first, count, out, s);
         case 2: return read_lanes<SF, 2>(a, map, first, count, out, s);
@@ -1541,7 +1544,7 @@ static void canon_force_lanes(const Arena& a, const CUtensorMap& map, cudaStream
 template <bool SF, int PASS>
 static void canon_force_pass(const Arena& a, const CUtensorMap& map, cudaStream_t s) {
 #if VLJ_LIST_STREAM
-    switch (lanes_for(a.nslots)) {
+    switch (lanes_of(a, a.nslots)) {
         case 8: return canon_force_lanes<SF, PASS, 8>(a, map, s);
         case 4: return canon_force_lanes<SF, PASS, 4>(a, map, s);
         case 2: return canon_force_lanes<SF, PASS, 2>(a, map, s);

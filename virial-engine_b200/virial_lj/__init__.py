@@ -521,8 +521,8 @@ class LennardJones:
         _check(_lib.vlj_debug_set_step_threads(self._h, int(threads)))
 
     def set_step_lanes(self, lanes):
-        """Lanes per particle of the step kernel: 0 by grid size, 1 or 2 (same
-        trajectory to the bit)."""
+        """Lanes per particle of the force passes: 0 by grid size, 1, 2, 4 or 8
+        (same results to the bit)."""
         _check(_lib.vlj_debug_set_step_lanes(self._h, int(lanes)))
 
     def set_tiles(self, on):
@@ -654,6 +654,10 @@ class Batch:
     def set_step_threads(self, threads):
         """Particles per block of the step kernel (64, 128 or 256)."""
         _check(_lib.vlj_debug_set_step_threads(self._sim(), int(threads)))
+
+    def set_step_lanes(self, lanes):
+        """Lanes per particle of the force passes: 0 by grid size, 1, 2, 4 or 8."""
+        _check(_lib.vlj_debug_set_step_lanes(self._sim(), int(lanes)))
 
     def set_graphs(self, on):
         _check(_lib.vlj_debug_set_graphs(self._sim(), int(bool(on))))
