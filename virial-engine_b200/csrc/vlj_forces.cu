@@ -22,9 +22,14 @@
 namespace vlj {
 
 constexpr uint32_t kTileBytes = kTileRows * kForceThreads * 16u;
-// Resident blocks per SM the step kernel's register budget is sized for.
+// Resident blocks of 128 per SM that the step kernel's register budget is sized
+// for: 64 registers at eight. Left to itself the compiler takes 66, which
+// leaves seven blocks of 128 and three of 256: 324 us against 300 so on 512
+// replicas at 128 particles a block and 362 against 306 at 256, 47.1 against
+// 46.2 and 53.3 against 45.5 on the 256,000-atom box (no spill). The form that
+// takes a heat-current sample needs more and has no such bound.
 #ifndef VLJ_STEP_MIN_BLOCKS
-#define VLJ_STEP_MIN_BLOCKS 1
+#define VLJ_STEP_MIN_BLOCKS 8
 #endif
 constexpr int kStepMinBlocks = VLJ_STEP_MIN_BLOCKS;
 // Lanes per particle of the force kernels, by grid size (lanes_for): at most
@@ -646,7 +651,7 @@ __device__ __forceinline__ uint32_t resident_neighbours(uint32_t b, uint32_t n, 
 // THREADS particles per block (Arena::step_threads, tuned per replica set
 // by virial_lj.tune_batch; the TMA tile ring needs kForceThreads).
 template <bool SHIFTED_FORCE, bool HEAT, int THREADS>
-__global__ void __launch_bounds__(THREADS, kStepMinBlocks) step_kernel(Arena a,
+__global__ void __launch_bounds__(THREADS, HEAT ? 1 : kStepMinBlocks * 128 / THREADS) step_kernel(Arena a,
                                                              const __grid_constant__ CUtensorMap map,
                                                              cudaGraphConditionalHandle next) {
     static_assert(VLJ_LIST_STREAM || THREADS == kForceThreads, "TMA tiles need kForceThreads");
