@@ -71,3 +71,14 @@ def test_scan_runs_at_their_edges(gpu, O, n):
     rng = np.random.default_rng(n)
     pos = rng.uniform(0.0, 1.0, (n, 3))
     run(gpu, O, pos, rng.uniform(0.002, 0.007, n), 1.0, 4)
+
+
+@pytest.mark.parametrize("cells", [1, 15, 16, 17, 25, 26])
+@pytest.mark.parametrize("n", [2, 5000])
+def test_scan_by_one_block_and_by_many(gpu, O, cells, n):
+    # 16^3 cells are one tile of the prefix sum; up to four tiles (25^3 cells)
+    # one block scans them all, beyond that a block each
+    rng = np.random.default_rng(cells)
+    radius = rng.uniform(0.3, 0.499, n) / cells
+    radius[0] = 0.4995 / cells
+    run(gpu, O, rng.uniform(0.0, 1.0, (n, 3)), radius, 1.0, 4)

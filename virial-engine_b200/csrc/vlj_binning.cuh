@@ -15,6 +15,7 @@
 #include <stdint.h>
 
 #include "vlj_place.h"
+#include "vlj_scan_shape.h"
 
 namespace vlj {
 namespace {
@@ -52,10 +53,8 @@ __global__ void nb_bin(const double* __restrict__ pos, BinGrid g, uint32_t* __re
 // nothing else uses before the scatter), and nb_scan adds up the totals before
 // its run and scans the run. One block for all cells spent its time waiting
 // for one load after another: 64^3 cells took it about 39 us, these two
-// launches take 5.8 us together.
-// `per` (a multiple of kScanTile) is the run: as many blocks as there are
-// tiles, but no more than places in `sorted`.
-constexpr uint32_t kScanTile = 4096;  // cells of one pass: four a thread
+// launches take 5.8 us together. Few cells are one run, which needs no sums
+// (bin_runs, which also gives the run's length `per`).
 
 __device__ __forceinline__ uint32_t nb_block_sum(uint32_t v, uint32_t* s_warp) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -211,12 +210,9 @@ inline cudaError_t enqueue_binning(const double* pos, const BinGrid& g, uint32_t
     if (e != cudaSuccess) return e;
     const unsigned blocks = (g.n + 255u) / 256u;
     nb_bin<<<blocks, 256, 0, s>>>(pos, g, cell_of, counts);
-    const uint64_t tiles = ((uint64_t)g.total + kScanTile - 1u) / kScanTile;
-    const uint64_t runs = tiles < g.n ? tiles : g.n;
-    const uint64_t per = (tiles + runs - 1u) / runs * kScanTile;
-    const unsigned scans = (unsigned)((g.total + per - 1u) / per);
-    nb_sums<<<scans, 1024, 0, s>>>(g, (uint32_t)per, counts, sorted);
-    nb_scan<<<scans, 1024, 0, s>>>(g, (uint32_t)per, sorted, counts, cell_start);
+    const BinRuns r = bin_runs(g.total, g.n);
+    if (bin_needs_sums(r)) nb_sums<<<r.blocks, 1024, 0, s>>>(g, r.per, counts, sorted);
+    nb_scan<<<r.blocks, 1024, 0, s>>>(g, r.per, sorted, counts, cell_start);
     nb_scatter<<<blocks, 256, 0, s>>>(g, cell_of, cell_start, counts, sorted);
     nb_order<<<(unsigned)(((uint64_t)g.total * 32u + 255u) / 256u), 256, 0, s>>>(
         g, cell_start, sorted, counts, g.total);

@@ -38,4 +38,28 @@ VLJ_HOST_DEVICE uint32_t scan_run(uint32_t chunks, uint32_t x, uint32_t least) {
     return even > least ? even : least;
 }
 
+// The stand-alone grid's scan (vlj_binning.cuh): blocks that take a run of
+// `per` cells each, whole tiles of kScanTile, and no more blocks than there are
+// particles (their sums lie in the order's buffer). Up to four tiles one block
+// takes them all, which needs no sums and so a launch less: 22.6 us against
+// 25.8 for a call over 4,913 cells, the same at 15,625, 27.8 against 25.8 at
+// 19,683. Beyond, a tile a block.
+constexpr uint32_t kScanTile = 4096;  // cells of one pass: four a thread
+constexpr uint32_t kOneBlockTiles = 4;
+
+struct BinRuns {
+    uint32_t per, blocks;
+};
+
+inline BinRuns bin_runs(uint32_t cells, uint32_t particles) {
+    const uint64_t tiles = ((uint64_t)cells + kScanTile - 1u) / kScanTile;
+    const uint64_t runs = tiles <= kOneBlockTiles ? 1u : (tiles < particles ? tiles : particles);
+    const uint64_t per = (tiles + runs - 1u) / runs * kScanTile;
+    return {(uint32_t)per, (uint32_t)((cells + per - 1u) / per)};
+}
+
+// Whether the blocks' sums are needed, a launch of their own: a single block
+// has nothing before its run.
+inline bool bin_needs_sums(const BinRuns& r) { return r.blocks > 1u; }
+
 }  // namespace vlj
