@@ -153,7 +153,9 @@ VLJ_API vlj_status vlj_measure(vlj_sim *sim, int *accepted);
 VLJ_API vlj_status vlj_poll(vlj_sim *sim, vlj_measurement *out, size_t capacity, size_t *written);
 VLJ_API vlj_status vlj_measure_now(vlj_sim *sim, vlj_measurement *out);
 
-/* ---- state: read_particles (lennard_jones.rs:1354-1374), in input order */
+/* ---- state: read_particles (lennard_jones.rs:1354-1374), in input order.
+ * Also refreshes the per-slot velocities and drawn values (vlj_velocities);
+ * it is no measurement: the measurement's sums stay as they were. */
 VLJ_API vlj_status vlj_read_particles(vlj_sim *sim, vlj_particle *out);
 /* Replaces every particle's position and velocity (a restart from a
  * snapshot); lists rebuild before the next force evaluation. No reference
@@ -172,7 +174,7 @@ VLJ_API vlj_status vlj_target_temperature(const vlj_sim *sim, int *has, double *
  * buffers; with no graphics interop these are plain device pointers:
  * positions as three f64 arrays (x, y, z) of `stride` elements each, in slot
  * order; velocities as float4 (vx, vy, vz, drawn value) per slot, written by
- * each measurement. */
+ * each measurement and each vlj_read_particles. */
 VLJ_API vlj_status vlj_positions(const vlj_sim *sim, const double **xyz, size_t *stride);
 VLJ_API vlj_status vlj_velocities(const vlj_sim *sim, const float **vel4);
 
@@ -276,7 +278,8 @@ VLJ_API vlj_status vlj_batch_step(vlj_batch *batch, uint32_t steps);
 VLJ_API vlj_status vlj_batch_run(vlj_batch *batch, uint64_t steps);
 /* One measurement per replica into out[replicas]; waits. */
 VLJ_API vlj_status vlj_batch_measure(vlj_batch *batch, vlj_measurement *out);
-/* Replica r's particles into out (its count), input order; waits. */
+/* Replica r's particles into out (its count), input order; waits. Of the
+ * per-slot velocities only that replica's are refreshed. */
 VLJ_API vlj_status vlj_batch_read_particles(vlj_batch *batch, size_t replica, vlj_particle *out);
 VLJ_API vlj_status vlj_batch_count(const vlj_batch *batch, size_t *replicas, uint64_t *particles);
 /* Replica r's box sides as the simulation uses them (rounded to f32). */
@@ -365,7 +368,7 @@ VLJ_API vlj_status vlj_debug_read_grid(vlj_sim *sim, uint32_t *sorted, uint32_t 
 VLJ_API vlj_status vlj_debug_force_rebuild(vlj_sim *sim);
 /* Per-slot halves of each particle's pair energy and virial from the last
  * measurement, as (hi, lo) f32 pairs whose exact sum is the value (2n each),
- * and the raw 64-bit fixed-point slots (8). */
+ * and the raw 64-bit fixed-point slots (8). Reading particles leaves them. */
 VLJ_API vlj_status vlj_debug_read_partials(vlj_sim *sim, float *pe_half, float *w_half,
                                            int64_t *raw_slots);
 /* Writes the word in which a kernel records a fault (0: none, 1: a wait that
@@ -376,8 +379,8 @@ VLJ_API vlj_status vlj_debug_set_fault(vlj_sim *sim, uint32_t code);
 VLJ_API vlj_status vlj_debug_launches(uint64_t *launches);
 /* Kernels of this simulation that ran on the device (waits). */
 VLJ_API vlj_status vlj_debug_kernels_executed(vlj_sim *sim, uint64_t *kernels);
-/* The last measurement's per-particle float4 (vx, vy, vz, drawn value), in
- * input order (n x 4 floats); waits. */
+/* The per-particle float4 (vx, vy, vz, drawn value) of the last measurement or
+ * read-back of the particles, in input order (n x 4 floats); waits. */
 VLJ_API vlj_status vlj_debug_read_vel4(vlj_sim *sim, float *out);
 /* 0: enqueue steps as direct launches instead of CUDA graphs. */
 VLJ_API vlj_status vlj_debug_set_graphs(vlj_sim *sim, int on);

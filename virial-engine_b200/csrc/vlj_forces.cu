@@ -633,8 +633,8 @@ __global__ void __launch_bounds__(kForceThreads) prime_kernel(Arena a,
 // kick together, then drifts: x += v dt (constant energy), or the Langevin
 // A-O-A: x += v dt/2; v = c1 v + c2 xi; x += v dt/2. State updates in f64.
 // The new position goes to the other cache copy (neighbours still read this
-// step's), and the largest squared displacement since the last list build
-// feeds the next step's rebuild decision.
+// step's), and a squared displacement since the last list build that is past
+// the trigger feeds the next step's rebuild decision.
 // The block's run of particles when the blocks that share an SM in the
 // first wave take neighbouring runs (VLJ_STEP_REMAP): the hardware hands out
 // blocks g, g + sms, g + 2 sms, ... to one SM in that wave, so within each

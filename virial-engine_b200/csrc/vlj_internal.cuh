@@ -151,7 +151,7 @@ struct Box {
 
 // Mutable per-box words.
 struct Control {
-    uint32_t max_disp;   // f32 bits of the largest squared displacement
+    uint32_t max_disp;   // f32 bits of the largest squared displacement past the trigger, else 0
     uint32_t rebuild;    // this step rebuilds
     uint32_t reorder;    // this rebuild also moves particles into cell order
     uint32_t rebuilds;   // rebuilds so far (lennard_jones.wgsl:299-305)
@@ -171,7 +171,7 @@ struct Global {
     unsigned long long kernels;  // kernels of this arena that ran
     uint32_t grid_every_step;    // 1: bin, scan, scatter and sort every step (one box)
     uint32_t work_front;         // Arena::work entries at its front: cells of kDenseCell or more
-    uint32_t work_back;          // entries at its back (work[ncells - 1 - k]): the other non-empty cells
+    uint32_t work_back;          // entries at its back (work[work_cap - 1 - k]): the other non-empty cells
     uint32_t next_build;         // next work entry the list build takes
     uint32_t blocks_done;        // step-kernel blocks finished (the last one decides)
     uint32_t rb_boxes;           // boxes that rebuild this step (Arena::rb_box)

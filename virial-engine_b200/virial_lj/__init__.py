@@ -559,7 +559,8 @@ class LennardJones:
         return n.value
 
     def read_vel4(self):
-        """The last measurement's (vx, vy, vz, drawn value) per particle, input order."""
+        """(vx, vy, vz, drawn value) per particle of the last measurement or
+        read_particles, input order."""
         out = np.zeros((self._n, 4), np.float32)
         _check(_lib.vlj_debug_read_vel4(self._h, _ffi.ptr(out)))
         return out
@@ -572,7 +573,8 @@ class LennardJones:
         _check(_lib.vlj_debug_set_fault(self._h, int(code)))
 
     def read_partials(self):
-        """(pe, w, raw): per-slot (hi, lo) halves of pair energy and virial."""
+        """(pe, w, raw) of the last measurement: per-slot (hi, lo) halves of
+        pair energy and virial, and the fixed-point sums."""
         pe = np.zeros((self._n, 2), np.float32)
         w = np.zeros((self._n, 2), np.float32)
         raw = np.zeros(8, np.int64)
