@@ -382,7 +382,7 @@ def run_slab(args, world, rank, stream, flush_l2):
                                          thermostat=vl.Langevin(SLAB["temperature"],
                                                                 SLAB["friction"], 11 + rank)),
                           stream=stream.cuda_stream)
-    # warmed in the calls that are timed; the 32nd captures the graph of their last four steps
+    # warmed in the calls that are timed; the 32nd captures the last of their graphs
     for _ in range(max(args.warmup, 33)):
         sim.step(SLAB["every"])
     sim.clear_profile()

@@ -313,8 +313,8 @@ vlj_status poll_ring(vlj_sim* s, vlj_measurement* out, size_t capacity, size_t* 
 }  // namespace
 
 vlj_sim::~vlj_sim() {
-    if (graph_chunk) cudaGraphExecDestroy(graph_chunk);
-    if (graph_short) cudaGraphExecDestroy(graph_short);
+    for (cudaGraphExec_t g : graph_chunk)
+        if (g) cudaGraphExecDestroy(g);
     if (graph_one) cudaGraphExecDestroy(graph_one);
     if (graph_one_tmpl) cudaGraphDestroy(graph_one_tmpl);
     if (graph_one_heat) cudaGraphExecDestroy(graph_one_heat);
@@ -1413,25 +1413,24 @@ vlj_status sim_enqueue_steps(vlj_sim* s, uint32_t steps) {
         for (uint32_t k = 0; k < steps; k++) TRY(step_direct(s));
         return VLJ_OK;
     }
-    // Whole graphs of 16 steps, then, once captured, of 4, then single steps.
-    // At 1,000 atoms a graph of 4 saves about 8 us over its steps one by one
-    // (a run of 4 steps: 72 us against 80, of 31: 610 against 625), but
-    // capturing costs about 65 us a step of the graph. So the graphs of 16 and
-    // of one step are captured when first needed, and the one of 4 in the call
+    // Whole graphs of 16 steps, then, once captured, one each of 8, 4 and 2,
+    // then single steps. A graph launch fewer saves 2 to 4 us, but capturing
+    // costs about 65 us a step of the graph. So the graphs of 16 and of one
+    // step are captured when first needed, and a remainder's graph in the call
     // by which it would have saved its price: a short-lived simulation, or one
-    // whose calls are of ever new lengths, captures 17 steps at most. (With
-    // graphs of 8 and 2 beside it, all captured when first needed, a first run
-    // of 31 steps took 2,780 us, 1,900 so; those two saved less than 3 us a call.)
-    for (; steps >= kGraphChunk; steps -= kGraphChunk) {
-        if (!s->graph_chunk) TRY(build_graph(s, kGraphChunk, &s->graph_chunk));
-        CUDA_TRY(cudaGraphLaunch(s->graph_chunk, s->stream));
-        s->one_ready = false;  // the chunk's last step leaves the decision open
-    }
-    if (steps >= kGraphShort && !s->graph_short && ++s->short_uses >= kShortUses)
-        TRY(build_graph(s, kGraphShort, &s->graph_short));
-    for (; steps >= kGraphShort && s->graph_short; steps -= kGraphShort) {
-        CUDA_TRY(cudaGraphLaunch(s->graph_short, s->stream));
-        s->one_ready = false;
+    // whose calls are of ever new lengths, captures 17 steps at most (with all
+    // of them captured when first needed a first run of 31 steps at 1,000 atoms
+    // took 2,700 us, 1,900 so).
+    for (int k = 0; k < kChunks; k++) {
+        const uint32_t count = kGraphChunk >> k;
+        if (steps >= count && !s->graph_chunk[k]) {
+            if (k > 0 && ++s->chunk_uses[k] < kChunkUses) continue;
+            TRY(build_graph(s, count, &s->graph_chunk[k]));
+        }
+        for (; steps >= count; steps -= count) {
+            CUDA_TRY(cudaGraphLaunch(s->graph_chunk[k], s->stream));
+            s->one_ready = false;  // the chunk's last step leaves the decision open
+        }
     }
     if (steps > 0 && !s->graph_one) {
         s->one_decide = nullptr;
@@ -1546,16 +1545,18 @@ vlj_status sim_grow_lists(vlj_sim* s, bool* grew) {
 }
 
 void sim_drop_step_graphs(vlj_sim* s) {
-    if (s->graph_chunk) cudaGraphExecDestroy(s->graph_chunk);
-    if (s->graph_short) cudaGraphExecDestroy(s->graph_short);
-    s->short_uses = 0;
+    for (int k = 0; k < kChunks; k++) {
+        if (s->graph_chunk[k]) cudaGraphExecDestroy(s->graph_chunk[k]);
+        s->graph_chunk[k] = nullptr;
+        s->chunk_uses[k] = 0;
+    }
     if (s->graph_one) cudaGraphExecDestroy(s->graph_one);
     if (s->graph_one_tmpl) cudaGraphDestroy(s->graph_one_tmpl);
     s->graph_one_tmpl = nullptr;
     s->one_decide = nullptr;
     s->one_ready = false;
     if (s->graph_one_heat) cudaGraphExecDestroy(s->graph_one_heat);
-    s->graph_chunk = s->graph_short = s->graph_one = s->graph_one_heat = nullptr;
+    s->graph_one = s->graph_one_heat = nullptr;
 }
 
 }  // namespace vlj

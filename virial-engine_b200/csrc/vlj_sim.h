@@ -14,10 +14,10 @@ namespace vlj {
 
 constexpr int kRing = 3;  // measurement read-back slots (lennard_jones.rs:320)
 constexpr uint32_t kGraphChunk = 16;  // most steps per graph launch
-constexpr uint32_t kGraphShort = 4;   // steps of the graph that takes what is left of a call
-// The call with such a rest in which that graph is captured (sim_enqueue_steps);
-// until then its steps go out one by one.
-constexpr uint32_t kShortUses = 32;
+constexpr int kChunks = 4;            // graphs of 16, 8, 4 and 2 steps
+// The call with a use for it in which a graph of 8, 4 or 2 steps is captured
+// (sim_enqueue_steps); until then its steps go out in smaller ones.
+constexpr uint32_t kChunkUses = 32;
 // Steps that a run enqueues at a time: whole graphs of 16.
 constexpr uint32_t kRunSteps = 12 * kGraphChunk;
 
@@ -93,14 +93,14 @@ struct vlj_sim {
     double* pin_x = nullptr;
     double* pin_v = nullptr;
     uint32_t* pin_id = nullptr;
-    // captured steps: graphs of kGraphChunk, kGraphShort and one steps, each
-    // step's rebuild chain under a conditional node; the short one is captured
-    // in the kShortUses-th call with a use for it, the others when first needed
+    // captured steps: graphs of kGraphChunk >> k steps and one of a single
+    // step, each step's rebuild chain under a conditional node; those of 16 and
+    // of one step captured when first needed, the others in the kChunkUses-th
+    // call with a use for them
     bool use_graphs = true;
     cudaStream_t capture_stream = nullptr;
-    cudaGraphExec_t graph_chunk = nullptr;
-    cudaGraphExec_t graph_short = nullptr;
-    uint32_t short_uses = 0;  // calls with a use for it since the graphs were last dropped
+    cudaGraphExec_t graph_chunk[vlj::kChunks] = {};
+    uint32_t chunk_uses[vlj::kChunks] = {};  // calls with a use for each since the last drop
     cudaGraphExec_t graph_one = nullptr;
     // graph_one's template (kept for node updates) and its decide node: while
     // the last step enqueued was graph_one's, whose step kernel took this
