@@ -10,12 +10,16 @@ import pytest
 pytestmark = pytest.mark.gpu
 
 BINS = 8
+ENSEMBLES = ["none", "langevin", "nose_hoover", "exchange"]
 
 
-def make(gpu, stream):
+def make(gpu, stream, ensemble):
     p = gpu.lattice(1000, 11.0, 1.0, 3)
-    sim = gpu.LennardJones(p, gpu.Settings([11.0] * 3, dt=0.004, profile_bins=BINS,
-                                           thermostat=gpu.Langevin(1.0, 1.0, 5)), stream=stream.cuda_stream)
+    t = {"langevin": gpu.Langevin(1.0, 1.0, 5), "nose_hoover": gpu.NoseHoover(1.0, 0.5)}.get(ensemble)
+    sim = gpu.LennardJones(p, gpu.Settings([11.0] * 3, dt=0.004, profile_bins=BINS, thermostat=t),
+                           stream=stream.cuda_stream)
+    if ensemble == "exchange":
+        sim.set_heat_exchange(gpu.HeatExchange((0.0, 1.0), (5.5, 6.5), 0.01))
     sim.set_graphs(False)
     sim.step(30)
     sim.sample_profile()
@@ -29,10 +33,11 @@ def profile(sim):
     return p.samples, np.array([[s.particles, *s.kinetic, *s.virial, s.potential] for s in p.slabs]).tobytes()
 
 
-def test_captured_sample_takes_the_decision_on_each_launch(gpu):
+@pytest.mark.parametrize("ensemble", ENSEMBLES)
+def test_captured_sample_takes_the_decision_on_each_launch(gpu, ensemble):
     import torch
     stream = torch.cuda.Stream()
-    sim = make(gpu, stream)
+    sim = make(gpu, stream, ensemble)
     graph = torch.cuda.CUDAGraph()
     with torch.cuda.graph(graph, stream=stream):
         sim.sample_profile()
@@ -41,7 +46,7 @@ def test_captured_sample_takes_the_decision_on_each_launch(gpu):
         graph.replay()
     got = profile(sim)
     sim.close()
-    twin = make(gpu, stream)
+    twin = make(gpu, stream, ensemble)
     twin.step(37)
     twin.sample_profile()
     want = profile(twin)
@@ -49,10 +54,11 @@ def test_captured_sample_takes_the_decision_on_each_launch(gpu):
     assert got == want
 
 
-def test_measurement_after_a_captured_step(gpu):
+@pytest.mark.parametrize("ensemble", ENSEMBLES)
+def test_measurement_after_a_captured_step(gpu, ensemble):
     import torch
     stream = torch.cuda.Stream()
-    sim = make(gpu, stream)
+    sim = make(gpu, stream, ensemble)
     graph = torch.cuda.CUDAGraph()
     with torch.cuda.graph(graph, stream=stream):
         sim.step(1)
@@ -63,7 +69,7 @@ def test_measurement_after_a_captured_step(gpu):
         got = sim.measure_now()
     q = sim.read_particles()
     sim.close()
-    twin = make(gpu, stream)
+    twin = make(gpu, stream, ensemble)
     for _ in range(33):
         twin.step(1)
         want = twin.measure_now()
