@@ -86,10 +86,15 @@ __device__ __forceinline__ bool narrow_box(const Box& bx) {
 // Arena::part_entries, in proportion to the SMs).
 // Every part stages the cell's candidates again, so no further than two
 // homes, and not at all where the cells fill the warps by themselves.
-__device__ __forceinline__ uint32_t part_homes(const Arena& a, bool narrow) {
-    const uint32_t slots = a.glob->rb_slots;
-    if (slots > kPartHomes * a.part_entries) return narrow ? kPartHomes : 0u;
+// The decision works it out (split_homes), once for all that ask.
+__device__ __forceinline__ uint32_t split_homes(const Arena& a, uint32_t slots) {
+    if (slots > kPartHomes * a.part_entries) return 0u;
     return min(kPartHomes, max(2u, (slots + a.part_entries - 1u) / a.part_entries));
+}
+
+__device__ __forceinline__ uint32_t part_homes(const Arena& a, bool narrow) {
+    const uint32_t per = a.glob->part_homes;
+    return per ? per : (narrow ? kPartHomes : 0u);
 }
 
 // Work-list entries of a cell of m particles, split by `per` homes.
@@ -239,6 +244,7 @@ __device__ __forceinline__ void decide_block(const Arena& a, cudaGraphConditiona
         a.rb_first[grid ? 1 : 0] = n;
         g->rb_boxes = grid ? 1u : 0u;
         g->rb_slots = n;
+        g->part_homes = split_homes(a, n);
         g->any = c.rebuild;
         if (set) cudaGraphSetConditional(handle, c.rebuild);
         return;
@@ -328,6 +334,7 @@ __device__ __forceinline__ void decide_block(const Arena& a, cudaGraphConditiona
         a.rb_first[s_cbox] = s_cslot;
         g->rb_boxes = s_cbox;
         g->rb_slots = s_cslot;
+        g->part_homes = split_homes(a, s_cslot);
         g->any = s_cbox ? 1u : 0u;
         if (set) cudaGraphSetConditional(handle, s_cbox ? 1u : 0u);
     }

@@ -179,6 +179,8 @@ struct Global {
     uint32_t heat_next;          // heat-current samples written to the series so far
     uint32_t decided;            // a step kernel took the next step's decision, not yet consumed
     uint32_t tiles_ready;        // the 16-bit tile lists match the box's bricks (a build wrote them)
+    uint32_t part_homes;         // home particles per work entry where every cell splits, else 0
+    uint32_t pad;
 };
 
 // Nose-Hoover state of a box (Tuckerman's splitting, lennard_jones.wgsl:309-397).
